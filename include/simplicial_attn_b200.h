@@ -81,6 +81,21 @@ int sa_backward(const sa_params* p, const void* q, const void* k1, const void* k
                 const void* v2, const void* o, const float* lse, const void* d_o, void* dq, void* dk1,
                 void* dk2, void* dv1, void* dv2, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same two calls with the status word in a place of its own: `status` is 16 bytes that the device can
+ * write and that start at zero, 16-byte aligned -- device memory, or pinned host memory
+ * (cudaHostAllocMapped), in which case the host reads {code, wait site, block, 0} after any
+ * synchronisation, with no copy and nothing to clear per call.  Calls may share one word; it keeps the
+ * report of a call that gave up until the host sets it back to zero.  The workspace's first 256 bytes are
+ * then unused, and `workspace` may be NULL where the size function returns no more than those.  No
+ * counterpart in the reference. */
+int sa_forward_status(const sa_params* p, const void* q, const void* k1, const void* k2, const void* v1,
+                      const void* v2, void* o, float* lse, void* workspace, size_t workspace_bytes, void* status,
+                      void* stream);
+int sa_backward_status(const sa_params* p, const void* q, const void* k1, const void* k2, const void* v1,
+                       const void* v2, const void* o, const float* lse, const void* d_o, void* dq, void* dk1,
+                       void* dk2, void* dv1, void* dv2, void* workspace, size_t workspace_bytes, void* status,
+                       void* stream);
+
 /* The same backward for callers that have no way to obtain a device workspace at the moment they
  * need the gradients.  Typical cases: a plugin that runs inside a host framework's memory-allocator
  * callback, where calling the allocator again would re-enter it or deadlock; a worker in a process

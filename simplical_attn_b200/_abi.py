@@ -18,7 +18,7 @@ SA_ALGO_AUTO, SA_ALGO_GENERAL, SA_ALGO_TCGEN05 = 0, 1, 2
 EXPORTS = ("sa_forward", "sa_backward", "sa_forward_workspace_size", "sa_backward_workspace_size", "sa_read_status",
            "sa_resolve_algo", "sa_strerror", "sa_version", "sa_kernel_launches", "sa_backward_static",
            "sa_backward_static_capacity", "sa_read_status_static", "sa_read_status_ex", "sa_set_wait_limit_ns",
-           "sa_selftest_wait_timeout", "sa_copy_rows_async")
+           "sa_selftest_wait_timeout", "sa_copy_rows_async", "sa_forward_status", "sa_backward_status")
 
 
 class Strides(ctypes.Structure):
@@ -90,6 +90,32 @@ def load():
     lib.sa_kernel_launches.restype = ctypes.c_uint64
     _lib = lib
     return lib
+
+
+_binding = None
+
+
+def binding():
+    """The torch binding (`binding/sa_torch.cpp`): the operator on tensors as one native call per direction."""
+    global _binding
+    if _binding is None:
+        load()                                 # the binding links against the library
+        path = _build.BINDING
+        if _build.have_host_compiler():
+            path = _build.build_binding()
+        elif not os.path.exists(path):
+            raise OSError(f"{path} is missing and there is no C++ compiler to build it")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("sa_torch", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.on_error(_raise)
+        _binding = mod
+    return _binding
+
+
+def _raise(fn: str, status: int, detail):
+    raise SimplicialAttnError(fn if detail is None else f"{fn} ({detail})", status)
 
 
 def strerror(status: int) -> str:

@@ -7,8 +7,10 @@ from __future__ import annotations
 import concurrent.futures
 import hashlib
 import os
+import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -84,7 +86,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(res.stdout + res.stderr)
     if any(res.returncode != 0 for _, res in results):
         raise RuntimeError("nvcc failed building " + LIB)
-    link = subprocess.run([nvcc, "-shared", "-o", LIB] + [obj for obj, _ in results], capture_output=True, text=True)
+    link = subprocess.run([nvcc, "-shared", "-Xlinker", "-soname=" + os.path.basename(LIB), "-o", LIB] + [obj for obj, _ in results], capture_output=True, text=True)
     if verbose or link.returncode != 0:
         sys.stderr.write(link.stdout + link.stderr)
     if link.returncode != 0:
@@ -94,5 +96,56 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+# ---- the torch binding: host code only, compiled by the C++ compiler against torch's headers
+BINDING_SRC = os.path.join(PKG, "binding", "sa_torch.cpp")
+BINDING = os.path.join(LIB_DIR, "sa_torch.so")
+BINDING_STAMP = BINDING + ".sources"
+CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
+CUDA_INCLUDE = os.path.join(os.path.dirname(os.path.dirname(nvcc_path())), "include")
+
+
+def cxx_path() -> str:
+    # the system compiler, not $CXX: one that links its own static libstdc++ breaks exceptions across torch's libraries
+    return "g++"
+
+
+def have_host_compiler() -> bool:
+    return shutil.which(cxx_path()) is not None and os.path.exists(CUDA_INCLUDE)
+
+
+def binding_digest() -> str:
+    import torch
+    h = hashlib.sha256(" ".join(CXX_FLAGS + [torch.__version__, sys.version]).encode())
+    for d in (BINDING_SRC, os.path.join(os.path.dirname(PKG), "include", "simplicial_attn_b200.h")):
+        with open(d, "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()
+
+
+def build_binding(force: bool = False) -> str:
+    """Compile the torch binding if it is missing or was built from other sources (or for another torch)."""
+    digest = binding_digest()
+    if not force and os.path.exists(BINDING) and os.path.exists(BINDING_STAMP):
+        with open(BINDING_STAMP) as f:
+            if f.read().strip() == digest:
+                return BINDING
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), CUDA_INCLUDE,
+           sysconfig.get_paths()["include"]]
+    cmd = ([cxx_path()] + CXX_FLAGS + [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-I" + d for d in inc]
+           + ["-o", BINDING, BINDING_SRC, LIB, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+              "-ltorch_python", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
+    os.makedirs(LIB_DIR, exist_ok=True)
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("the C++ compiler failed building " + BINDING)
+    with open(BINDING_STAMP, "w") as f:
+        f.write(digest + "\n")
+    return BINDING
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_binding(force="--force" in sys.argv))

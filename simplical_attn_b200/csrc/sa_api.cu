@@ -33,7 +33,12 @@ constexpr int kMaxChunks = 8;      // passes the library is willing to chain (wi
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 bool stride_ok8(const sa_strides& s) { return s.b % 8 == 0 && s.n % 8 == 0 && s.h % 8 == 0; }
 
-int elem_size(int dtype) { return dtype == SA_F32 ? 4 : 2; }
+// Whether the buffer can serve a call that needs `need` bytes, of which the first kStatusBytes are only used for
+// the status word: a call that needs nothing else takes no buffer at all.
+bool workspace_ok(const void* workspace, size_t bytes, size_t need) {
+    if (!workspace) return need <= kStatusBytes;
+    return bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0;
+}
 
 int validate(const sa_params* p) {
     if (!p) return SA_ERR_NULL_POINTER;
@@ -273,14 +278,9 @@ int plan_sm_count() {
     return n > 0 ? n : 148;
 }
 
-template <typename Kern>
-bool set_smem(Kern kern, int bytes) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-}
-
 template <bool F16>
 int launch_fwd_tc_t(const KParams& k, const void* q, const void* k1, const void* k2, const void* v1, const void* v2, void* o,
-                    float* lse, void* workspace, cudaStream_t st) {
+                    float* lse, sa::DeviceStatus* status, cudaStream_t st) {
     DeviceInfo& dev = device_info();
     if (dev.cc_major != 10) return SA_ERR_NOT_SM100;
     CUtensorMap map_k1, map_v1;
@@ -292,12 +292,12 @@ int launch_fwd_tc_t(const KParams& k, const void* q, const void* k1, const void*
     const int qpb = (sa::tc::kNumRowTiles * sa::tc::kRowTile) >> P.dw_log2;
     P.num_qblocks = (k.N + qpb - 1) / qpb;
     P.num_units = (long)k.B * k.H * P.num_qblocks;
-    P.status = reinterpret_cast<sa::DeviceStatus*>(workspace);
+    P.status = status;
     P.wait_limit_ns = g_wait_limit_ns.load();
     const long grid = P.num_units < dev.sm_count ? P.num_units : dev.sm_count;
     const bool has_bias = k.k2_bias != 0.f || k.v2_bias != 0.f;
     auto launch = [&](auto kern, int smem_bytes) {
-        if (!set_smem(kern, smem_bytes)) return false;
+        if (!sa::allow_dynamic_smem((const void*)kern, smem_bytes)) return false;
         kern<<<(unsigned)grid, sa::tc::kFwdThreads, smem_bytes, st>>>(P, map_k1, map_v1, (const __nv_bfloat16*)q,
                                                                        (const __nv_bfloat16*)k2, (const __nv_bfloat16*)v2,
                                                                        (__nv_bfloat16*)o, lse);
@@ -316,16 +316,16 @@ int launch_fwd_tc_t(const KParams& k, const void* q, const void* k1, const void*
 }
 
 int launch_fwd_tc_one(const sa_params* p, const KParams& k, const void* q, const void* k1, const void* k2, const void* v1,
-                      const void* v2, void* o, float* lse, void* workspace, cudaStream_t st) {
-    return p->dtype == SA_F16 ? launch_fwd_tc_t<true>(k, q, k1, k2, v1, v2, o, lse, workspace, st)
-                              : launch_fwd_tc_t<false>(k, q, k1, k2, v1, v2, o, lse, workspace, st);
+                      const void* v2, void* o, float* lse, sa::DeviceStatus* status, cudaStream_t st) {
+    return p->dtype == SA_F16 ? launch_fwd_tc_t<true>(k, q, k1, k2, v1, v2, o, lse, status, st)
+                              : launch_fwd_tc_t<false>(k, q, k1, k2, v1, v2, o, lse, status, st);
 }
 
 // One pass, or one pass per 128-position chunk of the K2 window merged into o / lse.
 int launch_fwd_tc(const sa_params* p, const KParams& k, const void* q, const void* k1, const void* k2, const void* v1,
-                  const void* v2, void* o, float* lse, void* workspace, cudaStream_t st) {
+                  const void* v2, void* o, float* lse, void* workspace, sa::DeviceStatus* status, cudaStream_t st) {
     const int nc = num_chunks(k);
-    if (nc == 1) return launch_fwd_tc_one(p, k, q, k1, k2, v1, v2, o, lse, workspace, st);
+    if (nc == 1) return launch_fwd_tc_one(p, k, q, k1, k2, v1, v2, o, lse, status, st);
     const ChunkTemps t = chunk_temps(k, false);
     uint8_t* base = static_cast<uint8_t*>(workspace) + kStatusBytes;
     void* o_t = base + t.o;
@@ -333,7 +333,7 @@ int launch_fwd_tc(const sa_params* p, const KParams& k, const void* q, const voi
     for (int c = 0; c < nc; ++c) {
         KParams kc = chunk_params(k, c);
         if (c > 0) kc.o = contiguous_strides(k.N, k.H, k.D);
-        const int rc = launch_fwd_tc_one(p, kc, q, k1, k2, v1, v2, c == 0 ? o : o_t, c == 0 ? lse : lse_t, workspace, st);
+        const int rc = launch_fwd_tc_one(p, kc, q, k1, k2, v1, v2, c == 0 ? o : o_t, c == 0 ? lse : lse_t, status, st);
         if (rc != SA_OK) return rc;
         if (c == 0) continue;
         const long total = (long)k.B * k.N * k.H * (k.D / 8);
@@ -364,10 +364,9 @@ size_t bwd_tc_kernel_workspace(const KParams& k) {
 // Returns an sa_status, or -1 when the tensor-core backward declines the problem (nothing has been launched then).
 int launch_bwd_tc(const sa_params* p, const KParams& k, const void* q, const void* k1, const void* k2, const void* v1,
                   const void* v2, const void* o, const float* lse, const void* d_o, void* dq, void* dk1, void* dk2, void* dv1,
-                  void* dv2, void* workspace, cudaStream_t st) {
+                  void* dv2, void* workspace, sa::DeviceStatus* status, cudaStream_t st) {
     const int nc = num_chunks(k);
     uint8_t* kernel_ws = static_cast<uint8_t*>(workspace) + kStatusBytes;
-    sa::DeviceStatus* status = reinterpret_cast<sa::DeviceStatus*>(workspace);
     const bool f16 = p->dtype == SA_F16;
     const ChunkTemps t = chunk_temps(k, true);
     uint8_t* temps = kernel_ws + bwd_tc_kernel_workspace(k);
@@ -524,9 +523,18 @@ int sa_forward(const sa_params* p, const void* q, const void* k1, const void* k2
                float* lse, void* workspace, size_t workspace_bytes, void* stream) {
     const int v = validate(p);
     if (v != SA_OK) return v;
-    if (!q || !k1 || !k2 || !v1 || !v2 || !o || !lse || !workspace) return SA_ERR_NULL_POINTER;
-    if (workspace_bytes < sa_forward_workspace_size(p) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
-        return SA_ERR_WORKSPACE;
+    if (!workspace) return SA_ERR_NULL_POINTER;
+    if (workspace_bytes < kStatusBytes) return SA_ERR_WORKSPACE;
+    return sa_forward_status(p, q, k1, k2, v1, v2, o, lse, workspace, workspace_bytes, workspace, stream);
+}
+
+int sa_forward_status(const sa_params* p, const void* q, const void* k1, const void* k2, const void* v1, const void* v2, void* o,
+                      float* lse, void* workspace, size_t workspace_bytes, void* status_word, void* stream) {
+    const int v = validate(p);
+    if (v != SA_OK) return v;
+    if (!q || !k1 || !k2 || !v1 || !v2 || !o || !lse || !status_word) return SA_ERR_NULL_POINTER;
+    if (!workspace_ok(workspace, workspace_bytes, sa_forward_workspace_size(p)) || !aligned16(status_word)) return SA_ERR_WORKSPACE;
+    sa::DeviceStatus* status = static_cast<sa::DeviceStatus*>(status_word);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const KParams k = make_kparams(p);
     int algo = resolve(p, false);
@@ -536,10 +544,9 @@ int sa_forward(const sa_params* p, const void* q, const void* k1, const void* k2
         if (p->algo == SA_ALGO_TCGEN05) return SA_ERR_BAD_STRIDE;
         algo = SA_ALGO_GENERAL;
     }
-    if (algo == SA_ALGO_TCGEN05) return launch_fwd_tc(p, k, q, k1, k2, v1, v2, o, lse, workspace, st);
+    if (algo == SA_ALGO_TCGEN05) return launch_fwd_tc(p, k, q, k1, k2, v1, v2, o, lse, workspace, status, st);
     const cudaError_t e = sa::general::launch_fwd(p->dtype, k, q, k1, k2, v1, v2, o, lse, st);
     g_launches += 1;
-    (void)elem_size;
     return e == cudaSuccess ? SA_OK : SA_ERR_LAUNCH;
 }
 
@@ -548,9 +555,19 @@ int sa_backward(const sa_params* p, const void* q, const void* k1, const void* k
                 void* workspace, size_t workspace_bytes, void* stream) {
     const int v = validate(p);
     if (v != SA_OK) return v;
-    if (!q || !k1 || !k2 || !v1 || !v2 || !o || !lse || !d_o || !workspace) return SA_ERR_NULL_POINTER;
-    if (workspace_bytes < sa_backward_workspace_size(p) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
-        return SA_ERR_WORKSPACE;
+    if (!workspace) return SA_ERR_NULL_POINTER;
+    if (workspace_bytes < kStatusBytes) return SA_ERR_WORKSPACE;
+    return sa_backward_status(p, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, workspace, workspace_bytes, workspace, stream);
+}
+
+int sa_backward_status(const sa_params* p, const void* q, const void* k1, const void* k2, const void* v1, const void* v2,
+                       const void* o, const float* lse, const void* d_o, void* dq, void* dk1, void* dk2, void* dv1, void* dv2,
+                       void* workspace, size_t workspace_bytes, void* status_word, void* stream) {
+    const int v = validate(p);
+    if (v != SA_OK) return v;
+    if (!q || !k1 || !k2 || !v1 || !v2 || !o || !lse || !d_o || !status_word) return SA_ERR_NULL_POINTER;
+    if (!workspace_ok(workspace, workspace_bytes, sa_backward_workspace_size(p)) || !aligned16(status_word)) return SA_ERR_WORKSPACE;
+    sa::DeviceStatus* status = static_cast<sa::DeviceStatus*>(status_word);
     if (!dq && !dk1 && !dk2 && !dv1 && !dv2) return SA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const KParams k = make_kparams(p);
@@ -564,7 +581,7 @@ int sa_backward(const sa_params* p, const void* q, const void* k1, const void* k
     }
     if (algo == SA_ALGO_TCGEN05) {
         if (device_info().cc_major != 10) return SA_ERR_NOT_SM100;
-        const int rc = launch_bwd_tc(p, k, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, workspace, st);
+        const int rc = launch_bwd_tc(p, k, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, workspace, status, st);
         if (rc != -1) return rc;      // -1: the tensor-core backward declines this problem
         if (p->algo == SA_ALGO_TCGEN05) return SA_ERR_UNSUPPORTED;
     }

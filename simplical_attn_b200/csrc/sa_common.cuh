@@ -7,6 +7,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+#include <vector>
+
 #include "../../include/simplicial_attn_b200.h"
 
 namespace sa {
@@ -25,8 +28,9 @@ struct KParams {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
-// Device status word kept in the first bytes of the caller's workspace.
-struct DeviceStatus {
+// Status word of a call: in the first bytes of the caller's workspace, or wherever the caller asked for it
+// (device memory or pinned host memory; 16-byte aligned, written with one store).
+struct alignas(16) DeviceStatus {
     int code;        // 0 or SA_ERR_DEVICE_TIMEOUT
     int where;       // id of the wait that gave up
     int block;       // block that recorded it
@@ -47,6 +51,22 @@ __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// Raises a kernel's limit of dynamic shared memory, once per kernel and device: the driver call takes longer than
+// a small kernel's launch.
+inline bool allow_dynamic_smem(const void* kern, int bytes) {
+    struct Entry { const void* kern; int device, bytes; };
+    static std::mutex mu;
+    static std::vector<Entry> done;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Entry& e : done)
+        if (e.kern == kern && e.device == device && e.bytes >= bytes) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    done.push_back({kern, device, bytes});
+    return true;
 }
 
 }  // namespace sa

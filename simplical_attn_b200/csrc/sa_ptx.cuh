@@ -54,7 +54,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // word in the caller's workspace.
 struct WaitCtx {
     volatile int* abort_flag;    // shared memory
-    DeviceStatus* status;        // global memory
+    DeviceStatus* status;        // global memory (or pinned host memory)
     uint64_t limit_ns;           // how long one wait may last before the block gives up
 };
 
@@ -141,11 +141,12 @@ __device__ __forceinline__ bool mbar_wait_impl(uint64_t* bar, uint32_t parity, c
             if (t0 == 0) t0 = now;
             else if (now - t0 > ctx.limit_ns) {
                 *ctx.abort_flag = 1;
-                if (atomicCAS(&ctx.status->code, 0, (int)SA_ERR_DEVICE_TIMEOUT) == 0) {
-                    ctx.status->where = where;
-                    ctx.status->block = (int)blockIdx.x;
-                }
-                __threadfence();
+                // One 16-byte store, so that a reader never sees half a report; of several blocks that give up at the
+                // same time the last one stays (the word may be host memory, where the first could not be kept with
+                // an atomic operation on every system).
+                if (*(volatile int*)&ctx.status->code == 0)
+                    *reinterpret_cast<int4*>(ctx.status) = make_int4((int)SA_ERR_DEVICE_TIMEOUT, where, (int)blockIdx.x, 0);
+                __threadfence_system();
                 return false;
             }
         }

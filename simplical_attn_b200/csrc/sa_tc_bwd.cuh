@@ -1806,15 +1806,13 @@ int launch_bwd_t(const KParams& k, const void* q, const void* k1, const void* k2
         if (k.D == 128) {
             auto kern = has_bias ? bwd_col_kernel<128, true, F16> : bwd_col_kernel<128, false, F16>;
             using LC = ColSmem<128>;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LC::kAlloc) != cudaSuccess)
-                return SA_ERR_LAUNCH;
+            if (!allow_dynamic_smem((const void*)kern, LC::kAlloc)) return SA_ERR_LAUNCH;
             kern<<<(unsigned)grid, kColThreads, LC::kAlloc, st>>>(P, m1, m2, bf(q), bf(k2), bf(v2), bf(d_o),
                                                                              (__nv_bfloat16*)dk1, (__nv_bfloat16*)dv1);
         } else {
             auto kern = has_bias ? bwd_col_kernel<64, true, F16> : bwd_col_kernel<64, false, F16>;
             using LC = ColSmem<64>;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LC::kAlloc) != cudaSuccess)
-                return SA_ERR_LAUNCH;
+            if (!allow_dynamic_smem((const void*)kern, LC::kAlloc)) return SA_ERR_LAUNCH;
             kern<<<(unsigned)grid, kColThreads, LC::kAlloc, st>>>(P, m1, m2, bf(q), bf(k2), bf(v2), bf(d_o),
                                                                             (__nv_bfloat16*)dk1, (__nv_bfloat16*)dv1);
         }
@@ -1834,7 +1832,7 @@ int launch_bwd_t(const KParams& k, const void* q, const void* k1, const void* k2
             int smem = k_ring + 1024 + 2 * ring_rows * (hd + 2) * 4 + extra;
             if (!need_kv2 || smem > max_dyn) { ring_rows = 0; smem = k_ring + 1024 + extra; }
             if (smem < k_min) smem = k_min;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn) != cudaSuccess) return false;
+            if (!allow_dynamic_smem((const void*)kern, max_dyn)) return false;
             kern<<<(unsigned)grid, threads, smem, st>>>(P, m1, m2, bf(q), bf(k2), bf(v2), bf(d_o), (__nv_bfloat16*)dq,
                                                         need_kv2, ring_rows);
             return true;

@@ -3,7 +3,9 @@
 Same names, argument meaning and return values as the reference's
 `simplicial/triton_impl.py` (`TwoSimplicialAttentionFunction`, :15-158; `TwoSimplicialAttention`,
 :161-186); the Triton launches are replaced by calls through the C ABI of
-libsimplicial_attn_b200.so.  torch supplies device memory and the current stream, nothing else.
+libsimplicial_attn_b200.so, made by a native binding (`binding/sa_torch.cpp`: argument checks, output
+allocation, autograd node) so that a small problem is not bound by Python.  torch supplies device memory
+and the current stream, nothing else.
 
 Additions that keep the reference call signature valid:
   * K/V may have fewer heads than Q (`H % Hkv == 0`); query head h reads KV head h // (H // Hkv).
@@ -39,28 +41,6 @@ def _ptr(t: Optional[torch.Tensor]):
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
-def _check_inputs(q, k1, k2, v1, v2, halo1, halo2):
-    if not q.is_cuda:
-        raise RuntimeError("simplical_attn_b200 runs on CUDA tensors only; there is no CPU path")
-    if q.dim() != 4:
-        raise ValueError("q must be [batch, seq_len, num_heads, head_dim]")
-    B, N, H, D = q.shape
-    if q.dtype not in _DTYPES:
-        raise TypeError(f"unsupported dtype {q.dtype}")
-    for name, t, halo in (("k1", k1, halo1), ("v1", v1, halo1), ("k2", k2, halo2), ("v2", v2, halo2)):
-        if t.dtype != q.dtype or t.device != q.device:
-            raise TypeError(f"{name} must match q's dtype and device")
-        if t.dim() != 4 or t.shape[0] != B or t.shape[1] != N + halo or t.shape[3] != D:
-            raise ValueError(f"{name} must be [batch, seq_len + halo, kv_heads, head_dim], got {tuple(t.shape)}")
-        if t.shape[2] != k1.shape[2] or H % t.shape[2] != 0:
-            raise ValueError("K/V tensors must share a head count that divides the query head count")
-    return B, N, H, k1.shape[2], D
-
-
-def _unit_inner(t: torch.Tensor) -> torch.Tensor:
-    return t if t.stride(-1) == 1 else t.contiguous()
-
-
 def _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo):
     B, N, H, D = q.shape
     p = _abi.Params()
@@ -79,21 +59,22 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
     return ws
 
 
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+_default_workspace = _workspace       # where `_workspace` is replaced its buffers are used; otherwise the binding allocates
 
 
 class _StatusWatch:
     """Surfaces device-side timeouts without a synchronisation per call.
 
-    After every launch the status word of the call's workspace is copied, stream-ordered, into a
-    pinned host slot and an event is recorded.  The next call on the same device looks at the slots
-    whose event has already completed (a non-blocking query) and raises if one of them holds an
-    error.  `flush()` synchronises and checks everything that is still pending."""
+    A call without a workspace of its caller's has its kernels report into a pinned host word, which the
+    binding looks at before every launch.  A caller's workspace carries the status word itself: after the
+    launch it is copied, stream-ordered, into a pinned host slot and an event is recorded.  `poll()` looks
+    at the slots whose event has already completed (a non-blocking query) and raises if one of them holds
+    an error.  `flush()` synchronises and checks everything that is still pending."""
 
     SLOTS = 32                      # pinned status slots per device, reused
 
     def __init__(self):
+        self.active = False         # a watched workspace's status is still to be looked at
         self._dev = {}              # device index -> (view of the pinned [SLOTS, 4] int32 slots, free slots, pending, stream, ...)
 
     def _state(self, index: int):
@@ -116,6 +97,7 @@ class _StatusWatch:
 
     def watch(self, ws: torch.Tensor, label: str, stream_handle=None) -> None:
         _, free, pending, side, small, events, host_ptr, small_ptr, side_handle, _ = self._state(ws.device.index)
+        self.active = True
         if not free:
             self.poll(ws.device, wait_oldest=True)
         i = free.pop()
@@ -148,6 +130,7 @@ class _StatusWatch:
             else:
                 keep.append((ev, i, label))
         pending[:] = keep
+        self.active = any(st[2] for st in self._dev.values())
         if bad is not None:
             raise _abi.SimplicialAttnError(f"{bad[0]} (device side: wait site {bad[2]}, block {bad[3]})", bad[1])
 
@@ -159,6 +142,11 @@ class _StatusWatch:
             indices = [d.index if d.index is not None else torch.cuda.current_device()]
         for index in indices:
             self.poll(torch.device("cuda", index), wait=True)
+        binding = _abi.binding()
+        for index in binding.devices():
+            if device is None or index in indices:
+                torch.cuda.synchronize(index)
+                binding.poll(index)
 
 
 _status_watch = _StatusWatch()
@@ -171,27 +159,30 @@ def check_device_status(device=None) -> None:
     _status_watch.flush(device)
 
 
+def _report(ws: Optional[torch.Tensor], label: str, device) -> None:
+    """What follows a launch: the status word of a caller's workspace is watched; in debug mode every call is
+    synchronised and checked at once."""
+    if ws is not None:
+        _status_watch.watch(ws, label)
+    if debug_device_status:
+        _status_watch.flush(device)
+
+
 def two_simplicial_attn_fwd_kernel(q, k1, k2, v1, v2, w1, w2, scale, k2_bias=0.0, v2_bias=0.0, halo1=0, halo2=0,
                                    algo=None):
     """Forward launch (the reference's kernel of the same name, `simplicial/kernels.py:11-171`).
     Returns (O, LSE) with LSE = log sum exp of the logits, fp32 [B, H, N] (the reference's `M`)."""
-    lib = _abi.load()
-    q, k1, k2, v1, v2 = (_unit_inner(t) for t in (q, k1, k2, v1, v2))
-    B, N, H, Hkv, D = _check_inputs(q, k1, k2, v1, v2, halo1, halo2)
-    _status_watch.poll(q.device)
-    o = torch.empty_like(q)                                   # triton_impl.py:23
-    lse = torch.empty((B, H, N), device=q.device, dtype=torch.float32)
-    p = _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo or default_algo)
-    ws = _workspace(lib.sa_forward_workspace_size(ctypes.byref(p)), q.device)
-    sh = torch.cuda.current_stream().cuda_stream
-    rc = lib.sa_forward(ctypes.byref(p), _ptr(q), _ptr(k1), _ptr(k2), _ptr(v1), _ptr(v2), _ptr(o), _ptr(lse), _ptr(ws),
-                        ws.numel(), ctypes.c_void_p(sh))
-    _abi.check("sa_forward", rc)
-    if debug_device_status:
-        _abi.check("sa_forward (device)", lib.sa_read_status(_ptr(ws), ctypes.c_void_p(sh)))
-    else:
-        _status_watch.watch(ws, "sa_forward", sh)
-    return o, lse
+    algo = algo or default_algo
+    ws = None
+    if _workspace is not _default_workspace:
+        p = _make_params(q, k1, k2, v1, v2, q, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo)
+        ws = _workspace(_abi.load().sa_forward_workspace_size(ctypes.byref(p)), q.device)
+    if _status_watch.active:
+        _status_watch.poll(q.device)
+    out = _abi.binding().forward(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo], ws)
+    if ws is not None or debug_device_status:
+        _report(ws, "sa_forward", q.device)
+    return out
 
 
 def two_simplicial_attn_bwd(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias=0.0, v2_bias=0.0, halo1=0, halo2=0,
@@ -199,24 +190,21 @@ def two_simplicial_attn_bwd(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bi
     """Backward launches (the reference's compute_D_kernel + two_simplicial_attn_bwd_kv1_kernel +
     two_simplicial_attn_bwd_kv2_kernel, `simplicial/kernels.py:175-571`).  Returns
     (dq, dk1, dk2, dv1, dv2), `None` where `need[i]` is false."""
-    lib = _abi.load()
-    q, k1, k2, v1, v2, o, d_o = (_unit_inner(t) for t in (q, k1, k2, v1, v2, o, d_o))
-    _check_inputs(q, k1, k2, v1, v2, halo1, halo2)
-    _status_watch.poll(q.device)
-    grads = [torch.empty_like(t) if n else None for t, n in zip((q, k1, k2, v1, v2), need)]
-    p = _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo or default_algo)
-    p.d_o = _strides(d_o)
-    p.dq, p.dk1, p.dk2, p.dv1, p.dv2 = (_strides(g) for g in grads)
-    ws = _workspace(lib.sa_backward_workspace_size(ctypes.byref(p)), q.device)
-    sh = torch.cuda.current_stream().cuda_stream
-    rc = lib.sa_backward(ctypes.byref(p), _ptr(q), _ptr(k1), _ptr(k2), _ptr(v1), _ptr(v2), _ptr(o), _ptr(lse), _ptr(d_o),
-                         *[_ptr(g) for g in grads], _ptr(ws), ws.numel(), ctypes.c_void_p(sh))
-    _abi.check("sa_backward", rc)
-    if debug_device_status:
-        _abi.check("sa_backward (device)", lib.sa_read_status(_ptr(ws), ctypes.c_void_p(sh)))
-    else:
-        _status_watch.watch(ws, "sa_backward", sh)
-    return tuple(grads)
+    algo = algo or default_algo
+    ws = None
+    if _workspace is not _default_workspace:
+        p = _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo)
+        p.d_o = _strides(d_o)
+        p.dq, p.dk1, p.dk2, p.dv1, p.dv2 = (_strides(t) for t in (q, k1, k2, v1, v2))
+        ws = _workspace(_abi.load().sa_backward_workspace_size(ctypes.byref(p)), q.device)
+    if _status_watch.active:
+        _status_watch.poll(q.device)
+    bits = sum(1 << i for i, n in enumerate(need) if n)
+    grads = _abi.binding().backward(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo],
+                                    bits, ws)
+    if ws is not None or debug_device_status:
+        _report(ws, "sa_backward", q.device)
+    return grads
 
 
 # When true every call synchronises and raises at once if a device-side bounded wait gave up; otherwise
@@ -265,11 +253,19 @@ class TwoSimplicialAttentionFunction(torch.autograd.Function):
         return grads + (None,) * 7
 
 
+def _attend(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1=0, halo2=0):
+    """The operator with its autograd history: the binding's native node, or, where every call has to be checked or
+    given a caller's buffers, `TwoSimplicialAttentionFunction`."""
+    if debug_device_status or _status_watch.active or _workspace is not _default_workspace:
+        return TwoSimplicialAttentionFunction.apply(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2)
+    return _abi.binding().attention(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[default_algo])
+
+
 def two_simplicial_attention(q, k1, k2, v1, v2, w1, w2, scale=None, k2_bias=0.0, v2_bias=0.0, halo1=0, halo2=0):
     """Functional form; `scale` defaults to 1/sqrt(head_dim) (`simplicial/triton_impl.py:169`)."""
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
-    return TwoSimplicialAttentionFunction.apply(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2)
+    return _attend(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2)
 
 
 class TwoSimplicialAttention(torch.nn.Module):
@@ -286,5 +282,4 @@ class TwoSimplicialAttention(torch.nn.Module):
         self.v2_bias = v2_bias
 
     def forward(self, q, k1, k2, v1, v2):
-        return TwoSimplicialAttentionFunction.apply(q, k1, k2, v1, v2, self.w1, self.w2, self.scale, self.k2_bias,
-                                                    self.v2_bias)
+        return _attend(q, k1, k2, v1, v2, self.w1, self.w2, self.scale, self.k2_bias, self.v2_bias)
