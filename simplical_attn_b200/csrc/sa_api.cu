@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(32) wait_timeout_probe_kernel(sa::DeviceStatus
         sa::ptx::fence_mbar_init();
     }
     __syncwarp();
-    const sa::ptx::WaitCtx ctx{&abort_flag, status, limit_ns};
+    const sa::ptx::WaitCtx ctx{sa::ptx::smem_u32(&abort_flag), status, limit_ns};
     sa::ptx::mbar_wait(&bar, 0, ctx, where);      // phase 0 never completes
     sa::ptx::mbar_wait(&bar, 0, ctx, where + 1);  // after the first wait gave up every later wait falls through
 }
@@ -278,41 +278,51 @@ int plan_sm_count() {
     return n > 0 ? n : 148;
 }
 
+template <int HD, bool BIAS, bool F16>
+int launch_fwd_tc_k(sa::tc::FwdTcParams& P, int sm_count, const void* q, const void* k1, const void* k2, const void* v1, const void* v2,
+                    void* o, float* lse, cudaStream_t st) {
+    const KParams& k = P.k;
+    const int smem = sa::tc::fwd_smem_plan<HD>(P);
+    const int win = sa::tc::fwd_window_rows(P.dw_log2, P.row_tiles), qrows = P.row_tiles * (sa::tc::kRowTile >> P.dw_log2);
+    CUtensorMap map_k1, map_v1, map_q, map_k2, map_v2;
+    if (!make_map(&map_k1, k1, k.B, k.n1, k.Hkv, k.D, k.k1, sa::tc::kColPiece, F16) ||
+        !make_map(&map_v1, v1, k.B, k.n1, k.Hkv, k.D, k.v1, sa::tc::kColPiece, F16) ||
+        !make_map(&map_q, q, k.B, k.N, k.H, k.D, k.q, qrows, F16) || !make_map(&map_k2, k2, k.B, k.n2, k.Hkv, k.D, k.k2, win, F16) ||
+        !make_map(&map_v2, v2, k.B, k.n2, k.Hkv, k.D, k.v2, win, F16))
+        return SA_ERR_BAD_STRIDE;
+    auto kern = sa::tc::fwd_tc_kernel<HD, BIAS, F16>;
+    if (!sa::allow_dynamic_smem((const void*)kern, 227 * 1024)) return SA_ERR_LAUNCH;
+    const int grid = P.num_units < sm_count ? P.num_units : sm_count;
+    kern<<<(unsigned)grid, sa::tc::kFwdThreads, smem, st>>>(P, map_k1, map_v1, map_q, map_k2, map_v2, (__nv_bfloat16*)o, lse);
+    g_launches += 1;
+    return cudaGetLastError() == cudaSuccess ? SA_OK : SA_ERR_LAUNCH;
+}
+
 template <bool F16>
 int launch_fwd_tc_t(const KParams& k, const void* q, const void* k1, const void* k2, const void* v1, const void* v2, void* o,
                     float* lse, sa::DeviceStatus* status, cudaStream_t st) {
     DeviceInfo& dev = device_info();
     if (dev.cc_major != 10) return SA_ERR_NOT_SM100;
-    CUtensorMap map_k1, map_v1;
-    if (!make_map(&map_k1, k1, k.B, k.n1, k.Hkv, k.D, k.k1, sa::tc::kSubTile, F16)) return SA_ERR_BAD_STRIDE;
-    if (!make_map(&map_v1, v1, k.B, k.n1, k.Hkv, k.D, k.v1, sa::tc::kSubTile, F16)) return SA_ERR_BAD_STRIDE;
     sa::tc::FwdTcParams P{};
     P.k = k;
-    P.dw_log2 = dw_log2_of(k.w2);
-    const int qpb = (sa::tc::kNumRowTiles * sa::tc::kRowTile) >> P.dw_log2;
-    P.num_qblocks = (k.N + qpb - 1) / qpb;
-    P.num_units = (long)k.B * k.H * P.num_qblocks;
+    P.dw_log2 = dw_log2_of(k.w2) < 2 ? 2 : dw_log2_of(k.w2);
+    P.row_tiles = sa::tc::kNumRowTiles;
+    auto count = [&] {
+        const int qpb = (P.row_tiles * sa::tc::kRowTile) >> P.dw_log2;
+        P.num_qblocks = (k.N + qpb - 1) / qpb;
+        return (long)k.B * k.H * P.num_qblocks;
+    };
+    // A problem that does not fill the multiprocessors with pairs of row tiles is cut into single ones.
+    if (count() <= dev.sm_count) P.row_tiles = 1;
+    const long units = count();
+    if (units > 0x7fffffffL - dev.sm_count) return SA_ERR_UNSUPPORTED;
+    P.num_units = (int)units;
     P.status = status;
     P.wait_limit_ns = g_wait_limit_ns.load();
-    const long grid = P.num_units < dev.sm_count ? P.num_units : dev.sm_count;
     const bool has_bias = k.k2_bias != 0.f || k.v2_bias != 0.f;
-    auto launch = [&](auto kern, int smem_bytes) {
-        if (!sa::allow_dynamic_smem((const void*)kern, smem_bytes)) return false;
-        kern<<<(unsigned)grid, sa::tc::kFwdThreads, smem_bytes, st>>>(P, map_k1, map_v1, (const __nv_bfloat16*)q,
-                                                                       (const __nv_bfloat16*)k2, (const __nv_bfloat16*)v2,
-                                                                       (__nv_bfloat16*)o, lse);
-        return true;
-    };
-    bool ok;
-    if (k.D == 128)
-        ok = has_bias ? launch(sa::tc::fwd_tc_kernel<128, true, F16>, sa::tc::FwdSmem<128>::kAlloc)
-                      : launch(sa::tc::fwd_tc_kernel<128, false, F16>, sa::tc::FwdSmem<128>::kAlloc);
-    else
-        ok = has_bias ? launch(sa::tc::fwd_tc_kernel<64, true, F16>, sa::tc::FwdSmem<64>::kAlloc)
-                      : launch(sa::tc::fwd_tc_kernel<64, false, F16>, sa::tc::FwdSmem<64>::kAlloc);
-    if (!ok) return SA_ERR_LAUNCH;
-    g_launches += 1;
-    return cudaGetLastError() == cudaSuccess ? SA_OK : SA_ERR_LAUNCH;
+    auto go = [&](auto fn) { return fn(P, dev.sm_count, q, k1, k2, v1, v2, o, lse, st); };
+    if (k.D > 64) return has_bias ? go(launch_fwd_tc_k<128, true, F16>) : go(launch_fwd_tc_k<128, false, F16>);
+    return has_bias ? go(launch_fwd_tc_k<64, true, F16>) : go(launch_fwd_tc_k<64, false, F16>);
 }
 
 int launch_fwd_tc_one(const sa_params* p, const KParams& k, const void* q, const void* k1, const void* k2, const void* v1,

@@ -31,9 +31,16 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+// The functions with a template argument take a barrier as a 32-bit shared-memory address plus a constant: the
+// constant goes into the instruction, so a role that uses many barriers holds one register for all of them.
+template <int OFF>
+__device__ __forceinline__ void mbar_arrive(uint32_t base) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0+%1];" ::"r"(base), "n"(OFF) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) { mbar_arrive_expect_tx(smem_u32(bar), bytes); }
 // One probe of the barrier.  The suspend-time hint lets the hardware park the warp until the phase
 // completes (it wakes at once when it does) instead of spinning through issue slots that the
 // working warps of the same scheduler need.
@@ -49,11 +56,42 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+template <int OFF>
+__device__ __forceinline__ bool mbar_try_wait(uint32_t base, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1+%4], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(base), "r"(parity), "r"(20000u), "n"(OFF)
+        : "memory");
+    return ok != 0;
+}
+// Whether the phase with the given parity has completed, without waiting.
+template <int OFF>
+__device__ __forceinline__ bool mbar_test(uint32_t base, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1+%3], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(base), "r"(parity), "n"(OFF)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t lds_volatile(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
 // Shared by every wait of a block: once any wait has given up, all later waits return at once so
 // that the block drains, frees its tensor memory and exits.  `status` points at the DeviceStatus
 // word in the caller's workspace.
 struct WaitCtx {
-    volatile int* abort_flag;    // shared memory
+    uint32_t abort_flag;         // shared-memory address of an int
     DeviceStatus* status;        // global memory (or pinned host memory)
     uint64_t limit_ns;           // how long one wait may last before the block gives up
 };
@@ -115,42 +153,48 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;   // default limit, 2 s: far be
 
 // Waits for the phase with the given parity.  Bounded: after ctx.limit_ns it records where it gave
 // up, raises the block's abort flag and returns false.
-__device__ __forceinline__ bool mbar_wait_impl(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where);
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
+template <typename Probe>
+__device__ __forceinline__ bool mbar_wait_on(Probe probe, const WaitCtx& ctx, int where) {
 #ifdef SA_PROFILE
-    const long long t0 = clock64();
-    const bool r = mbar_wait_impl(bar, parity, ctx, where);
-    if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) {
-        atomicAdd(&g_prof_cycles[where & 63], (unsigned long long)(clock64() - t0));
-        atomicAdd(&g_prof_count[where & 63], 1ull);
-    }
-    return r;
+    const long long c0 = clock64();
+    auto done = [&](bool r) {
+        if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) {
+            atomicAdd(&g_prof_cycles[where & 63], (unsigned long long)(clock64() - c0));
+            atomicAdd(&g_prof_count[where & 63], 1ull);
+        }
+        return r;
+    };
 #else
-    return mbar_wait_impl(bar, parity, ctx, where);
+    auto done = [](bool r) { return r; };
 #endif
-}
-__device__ __forceinline__ bool mbar_wait_impl(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (probe()) return done(true);
     uint64_t t0 = 0;
     uint32_t spins = 0;
     while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*ctx.abort_flag) return false;
+        if (probe()) return done(true);
+        if (lds_volatile(ctx.abort_flag)) return done(false);
         if ((++spins & 0xff) == 0) {
             const uint64_t now = globaltimer_ns();
             if (t0 == 0) t0 = now;
             else if (now - t0 > ctx.limit_ns) {
-                *ctx.abort_flag = 1;
+                asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(ctx.abort_flag), "r"(1u) : "memory");
                 // One 16-byte store, so that a reader never sees half a report; of several blocks that give up at the
                 // same time the last one stays (the word may be host memory, where the first could not be kept with
                 // an atomic operation on every system).
                 if (*(volatile int*)&ctx.status->code == 0)
                     *reinterpret_cast<int4*>(ctx.status) = make_int4((int)SA_ERR_DEVICE_TIMEOUT, where, (int)blockIdx.x, 0);
                 __threadfence_system();
-                return false;
+                return done(false);
             }
         }
     }
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
+    return mbar_wait_on([&] { return mbar_try_wait(bar, parity); }, ctx, where);
+}
+template <int OFF>
+__device__ __forceinline__ bool mbar_wait(uint32_t base, uint32_t parity, const WaitCtx& ctx, int where) {
+    return mbar_wait_on([&] { return mbar_try_wait<OFF>(base, parity); }, ctx, where);
 }
 
 // Per-warpgroup register re-allocation: the data-movement warps give registers up, the softmax /
@@ -178,13 +222,36 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 // Coordinates are (d, row, head, batch); d * 2 bytes must be a multiple of 16.
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
+__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
                                             int c2, int c3) {
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2),
+        ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
         "r"(c3)
         : "memory");
+}
+
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
+    tma_load_4d(smem_u32(smem_dst), map, smem_u32(bar), c0, c1, c2, c3);
+}
+
+// Shared-memory accesses by 32-bit address.
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float lds_f32(uint32_t addr) { return __uint_as_float(lds32(addr)); }
+__device__ __forceinline__ void sts_f32(uint32_t addr, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -214,6 +281,15 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
                  : "memory");
 }
 // The same, issued by the elected lane of a convergent warp only.
+template <int OFF>
+__device__ __forceinline__ void tc_commit(uint32_t leader, uint32_t base) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0+%2];\n\t}"
+        ::"r"(base), "r"(leader), "n"(OFF)
+        : "memory");
+}
 __device__ __forceinline__ void tc_commit(uint32_t leader, uint64_t* bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
@@ -250,6 +326,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
         : "r"(addr)
         : "memory");
 }
+// 64 columns of 16 lanes (the address's lane and the next 15): thread t gets, for j = 0..7, columns 8j + 2 (t % 4) and the
+// next one of lane t / 4 in v[4j], v[4j + 1] and of lane t / 4 + 8 in v[4j + 2], v[4j + 3].
+__device__ __forceinline__ void tmem_ld_16x256_x8(uint32_t addr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(addr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -271,6 +360,20 @@ __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]
         "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
         "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
+}
+
+// N columns of the thread's own lane (N = 16 or 32), N packed words (8 or 16).
+template <int N>
+__device__ __forceinline__ void tmem_ld_n(uint32_t addr, uint32_t (&v)[N]) {
+    static_assert(N == 16 || N == 32, "widths the softmax uses");
+    if constexpr (N == 16) tmem_ld16(addr, v);
+    else tmem_ld32(addr, v);
+}
+template <int N>
+__device__ __forceinline__ void tmem_st_n(uint32_t addr, const uint32_t (&v)[N]) {
+    static_assert(N == 8 || N == 16, "widths the softmax uses");
+    if constexpr (N == 8) tmem_st8(addr, v);
+    else tmem_st16(addr, v);
 }
 
 // ----------------------------------------------------------------------------------------------

@@ -295,7 +295,7 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
     uint64_t* acc_free = sdp_ready + 5;               // dV1, dK1 read out (256 arrivals)
     uint32_t* tmem_slot = (uint32_t*)(smem + L::kMisc);
     volatile int* abort_flag = (volatile int*)(smem + L::kMisc + 4);
-    const WaitCtx wctx{abort_flag, P.status, P.wait_limit_ns};
+    const WaitCtx wctx{smem_u32((const void*)abort_flag), P.status, P.wait_limit_ns};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     SA_PROF_T0(t_life);
@@ -721,7 +721,7 @@ bwd_row_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
     const BwdBars B = bwd_bars<NS>((uint64_t*)(smem + L::kBars));
     uint32_t* tmem_slot = (uint32_t*)(smem + L::kMisc);
     volatile int* abort_flag = (volatile int*)(smem + L::kMisc + 4);
-    const WaitCtx wctx{abort_flag, P.status, P.wait_limit_ns};
+    const WaitCtx wctx{smem_u32((const void*)abort_flag), P.status, P.wait_limit_ns};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     SA_PROF_T0(t_life);
@@ -1195,7 +1195,7 @@ bwd_row2_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ C
     uint8_t* const stage_base = smem + L::kRing + 2 * ring_rows * (HD + 2) * 4 + 2048;      // behind the rings and the partial dQ rows
     uint32_t* tmem_slot = (uint32_t*)(smem + L::kMisc);
     volatile int* abort_flag = (volatile int*)(smem + L::kMisc + 4);
-    const WaitCtx wctx{abort_flag, P.status, P.wait_limit_ns};
+    const WaitCtx wctx{smem_u32((const void*)abort_flag), P.status, P.wait_limit_ns};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     SA_PROF_T0(t_life);
