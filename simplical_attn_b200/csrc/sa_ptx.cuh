@@ -153,8 +153,8 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;   // default limit, 2 s: far be
 
 // Waits for the phase with the given parity.  Bounded: after ctx.limit_ns it records where it gave
 // up, raises the block's abort flag and returns false.
-template <typename Probe>
-__device__ __forceinline__ bool mbar_wait_on(Probe probe, const WaitCtx& ctx, int where) {
+template <typename Test, typename Probe>
+__device__ __forceinline__ bool mbar_wait_on(Test test, Probe probe, const WaitCtx& ctx, int where) {
 #ifdef SA_PROFILE
     const long long c0 = clock64();
     auto done = [&](bool r) {
@@ -167,7 +167,7 @@ __device__ __forceinline__ bool mbar_wait_on(Probe probe, const WaitCtx& ctx, in
 #else
     auto done = [](bool r) { return r; };
 #endif
-    if (probe()) return done(true);
+    if (test()) return done(true);
     uint64_t t0 = 0;
     uint32_t spins = 0;
     while (true) {
@@ -190,11 +190,11 @@ __device__ __forceinline__ bool mbar_wait_on(Probe probe, const WaitCtx& ctx, in
     }
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, int where) {
-    return mbar_wait_on([&] { return mbar_try_wait(bar, parity); }, ctx, where);
+    return mbar_wait_on([&] { return mbar_test<0>(smem_u32(bar), parity); }, [&] { return mbar_try_wait(bar, parity); }, ctx, where);
 }
 template <int OFF>
 __device__ __forceinline__ bool mbar_wait(uint32_t base, uint32_t parity, const WaitCtx& ctx, int where) {
-    return mbar_wait_on([&] { return mbar_try_wait<OFF>(base, parity); }, ctx, where);
+    return mbar_wait_on([&] { return mbar_test<OFF>(base, parity); }, [&] { return mbar_try_wait<OFF>(base, parity); }, ctx, where);
 }
 
 // Per-warpgroup register re-allocation: the data-movement warps give registers up, the softmax /
@@ -446,6 +446,38 @@ __device__ __forceinline__ void mma_ts(uint32_t leader, uint32_t d_tmem, uint32_
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
         : "memory");
+}
+
+// The same with the low words of the descriptors plus a constant: the high words are constants (kDescHiK for K-major,
+// kDescHiMn), so an issuer loop holds one 32-bit register per operand instead of a 64-bit one per operand and step.
+constexpr uint32_t kDescHi = (uint32_t)((((uint64_t)(1024u >> 4)) << 32 | kDescVersion | kDescSwizzle128) >> 32);
+template <int OFFA, int OFFB>
+__device__ __forceinline__ void mma_ss_lo(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 x, y;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "add.u32 x, %1, %7;\n\tadd.u32 y, %2, %8;\n\t"
+        "mov.b64 da, {x, %6};\n\tmov.b64 db, {y, %6};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader), "n"(kDescHi), "n"(OFFA), "n"(OFFB)
+        : "memory");
+}
+template <int OFFA, int OFFB>
+__device__ __forceinline__ void mma_ts_lo(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 x, y;\n\t.reg .b64 db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "add.u32 x, %1, %7;\n\tadd.u32 y, %2, %8;\n\t"
+        "mov.b64 db, {y, %6};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [x], db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader), "n"(kDescHi), "n"(OFFA), "n"(OFFB)
+        : "memory");
+}
+// Low word of a K-major (lbo 16) or MN-major (lbo: bytes between 64-element slabs) descriptor.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+    return ((smem_addr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

@@ -17,7 +17,7 @@
 //
 // Warps.  0-3 / 4-7: softmax group of row tile 0 / 1.  8-11 / 12-15: auxiliary group of row tile 0 / 1: forms the A tile
 // of the next unit as soon as the tensor cores have read the current one, and merges the finished unit's delta rows,
-// both out of raw Q / K2 / V2 rows that are in shared memory by then.  16, 17: MMA issuers of row tile 0 and 1; their
+// both out of raw Q / K2 / V2 rows that are in shared memory by then.  16: MMA issuer; its
 // loop runs over the column tiles of all units without a break, so S of the next unit's first tile is computed while
 // the auxiliary group reads the finished T.  18: TMA loads of K1 / V1 (one ring of 128-row buffers, K1 and V1 in
 // turn).  19: TMA loads of the raw rows, a unit ahead.
@@ -157,6 +157,14 @@ struct RingPos {
     }
 };
 
+template <int N, typename F, int I = 0>
+__device__ __forceinline__ void static_for(F&& f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        static_for<N, F, I + 1>(static_cast<F&&>(f));
+    }
+}
+
 // BIAS = false: both biases are zero, every bias add folds away.  F16: the tensors are IEEE half instead of bf16
 // (same kernels; only the element encoding and the MMA's operand format differ).  The head dim may be smaller than
 // HD (a multiple of 8): TMA fills the missing columns with zeros and they are not written out.
@@ -184,16 +192,15 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
     constexpr int kStReady = kTFree + 16;                        //            m, l of the unit stored (softmax group -> auxiliary group)
     constexpr int kStFree = kStReady + 16;                       //            m, l consumed (auxiliary group -> softmax group)
     constexpr int kSReady = kStFree + 16;                        //            S tile computed (MMA warp -> softmax group)
-    constexpr int kP0Ready = kSReady + 16;                       //            P of columns 0..63 stored (softmax group -> MMA warp)
-    constexpr int kP1Ready = kP0Ready + 16;                      //            P of the rest stored
-    constexpr int kQkFull = kP1Ready + 16;                       // raw Q and K2 rows landed
+    constexpr int kPReady = kSReady + 16;                        //            P stored (softmax group -> MMA warp)
+    constexpr int kQkFull = kPReady + 16;                        // raw Q and K2 rows landed
     constexpr int kQkFree = kQkFull + 8;                         //             ... read by the auxiliary groups
     constexpr int kV2Full = kQkFree + 8;                         // raw V2 rows landed
     constexpr int kV2Free = kV2Full + 8;                         //             ... read by the auxiliary groups
     static_assert(kV2Free + 8 <= L::kMisc, "room for the barriers");
     uint32_t* tmem_base_slot = (uint32_t*)(smem + L::kMisc);
     volatile int* abort_flag = (volatile int*)(smem + L::kMisc + 4);
-    const WaitCtx wctx{smem_u32((const void*)abort_flag), P.status, P.wait_limit_ns};
+    const WaitCtx wctx{smem_base + L::kMisc + 4, P.status, P.wait_limit_ns};
 
     const int tid = threadIdx.x;
     SA_PROF_T0(t_life);
@@ -215,8 +222,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
         init(kStReady, 2, 4);
         init(kStFree, 2, 4);
         init(kSReady, 2, 1);
-        init(kP0Ready, 2, 4);
-        init(kP1Ready, 2, 4);
+        init(kPReady, 2, 4);
         init(kQkFull, 1, 1);
         init(kQkFree, 1, 4 * P.row_tiles);
         init(kV2Full, 1, 1);
@@ -322,79 +328,93 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                 }
             }
             __syncwarp();
-        } else if (warp - 16 < P.row_tiles) {
-            // -------------------------------------------------------------- MMA issuer of row tile r
-            const int r = warp - 16;
-            const uint32_t rb = smem_base + r * 8;
+        } else if (warp == 16) {
+            // -------------------------------------------------------------- MMA issuer: P.V and the next S of row tile 0, then of row
+            // tile 1, and so on.  The fixed order keeps the row tiles half a period apart.  (With an issuer of its own
+            // for each, their MMAs interleave, both S tiles are complete at the same time and both softmaxes run at
+            // the same time while the tensor cores idle.)
             const uint32_t leader = elect_one();      // the whole warp runs the loop; one lane issues
-            const uint32_t tm_s = tmem_base + r * kColTile, tm_t = tmem_t0 + r * HD;
-            RingPos g;                                // buffers are consumed in the order K1, V1, K1, V1, ...
-            // S tile = A . K1^T.  The columns are free: the P.V MMAs that read them were issued by this warp before, and
-            // the tensor cores run in order.
-            auto issue_s = [&](bool last, int width) {
-                mbar_wait<kFull>(smem_base + g.s * 8, g.phase, wctx, 3);
-                tc_fence_after();
+            const int nrt = P.row_tiles;
+            // S tile = A . K1^T into the columns that row tile r's last P.V MMAs read (issued before, and the tensor cores
+            // run in order)
+            auto issue_s = [&](int r, int buf, bool last, int width) {
                 const uint32_t idesc = make_idesc(128, width, false, false, F16);
-                const uint64_t da = desc_kmajor(smem_base + L::kA + r * L::kTileBytes, 0);
-                const uint64_t db = desc_kmajor(smem_base + L::kRing + g.s * L::kStageBytes, 0);
-#pragma unroll
-                for (int kk = 0; kk < HD / 16; ++kk) {
-                    const uint32_t off = ((kk >> 2) * L::kSlabBytes + (kk & 3) * 32) >> 4;
-                    mma_ss(leader, tm_s, da + off, db + off, idesc, kk > 0);
-                }
-                tc_commit<kSReady>(leader, rb);
-                tc_commit<kEmpty>(leader, smem_base + g.s * 8);
-                if (last) tc_commit<kAFree>(leader, rb);       // the A tile may be overwritten
-                g.next(P.stages);
+                const uint32_t da = desc_lo(smem_base + L::kA + r * L::kTileBytes, 16);
+                const uint32_t db = desc_lo(smem_base + L::kRing + buf * L::kStageBytes, 16);
+                static_for<HD / 16>([&](auto kk_c) {
+                    constexpr int kk = decltype(kk_c)::value, off = ((kk >> 2) * L::kSlabBytes + (kk & 3) * 32) >> 4;
+                    mma_ss_lo<off, off>(leader, tmem_base + r * kColTile, da, db, idesc, kk > 0);
+                });
+                SA_TR(0, 32 + 100 * r);
+                tc_commit<kSReady>(leader, smem_base + r * 8);
+                tc_commit<kEmpty>(leader, smem_base + buf * 8);
+                if (last) tc_commit<kAFree>(leader, smem_base + r * 8);       // the A tile may be overwritten
             };
+            RingPos g;                                // buffers are consumed in the order K1, V1, K1, V1, ...
             uint32_t n = 0, nu = 0;                   // column tiles, units so far
             UnitWalk w(P);
             UnitGeom ug = w.geom(P);
             if (w.valid(P)) {
-                mbar_wait<kAReady>(rb, 0, wctx, 4);
-                issue_s(ug.ntile == 1, ug.ntile == 1 ? ug.last_width : kColTile);
+                mbar_wait<kFull>(smem_base + g.s * 8, g.phase, wctx, 3);
+                for (int r = 0; r < nrt; ++r) {
+                    mbar_wait<kAReady>(smem_base + r * 8, 0, wctx, 4);
+                    tc_fence_after();
+                    issue_s(r, g.s, ug.ntile == 1, ug.ntile == 1 ? ug.last_width : kColTile);
+                }
+                g.next(P.stages);
             }
             while (w.valid(P)) {
+                UnitWalk wn = w;
+                wn.next(P);
+                const bool more = wn.valid(P);
+                const UnitGeom ng = more ? wn.geom(P) : ug;
+#pragma unroll 1
                 for (int t = 0; t < ug.ntile; ++t, ++n) {
                     const bool last = t == ug.ntile - 1;
                     const int ksteps = last ? ug.last_width / 16 : kColTile / 16;
-                    const uint32_t idesc = make_idesc(128, HD, false, true, F16);
-                    const uint64_t db = desc_mnmajor(smem_base + L::kRing + g.s * L::kStageBytes, L::kStageSlab);
-                    mbar_wait<kFull>(smem_base + g.s * 8, g.phase, wctx, 6);
-                    // the previous unit's T has been read out by the auxiliary group
-                    if (t == 0 && nu > 0) mbar_wait<kTFree>(rb, (nu - 1) & 1, wctx, 10);
-                    mbar_wait<kP0Ready>(rb, n & 1, wctx, 5);
-                    SA_TR(r, 20);
-                    tc_fence_after();
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        if (kk < ksteps) mma_ts(leader, tm_t, tm_s + kk * 8, db + kk * (2048 >> 4), idesc, t > 0 || kk > 0);
-                    mbar_wait<kP1Ready>(rb, n & 1, wctx, 7);
-                    SA_TR(r, 21);
-                    tc_fence_after();
-#pragma unroll
-                    for (int kk = 4; kk < 8; ++kk)
-                        if (kk < ksteps) mma_ts(leader, tm_t, tm_s + kk * 8, db + kk * (2048 >> 4), idesc, true);
-                    tc_commit<kEmpty>(leader, smem_base + g.s * 8);
-                    if (last) tc_commit<kOReady>(leader, rb);
+                    const bool have_next = !last || more;                      // the next S tile, which may be the next unit's first
+                    const bool nlast = last ? ng.ntile == 1 : t + 1 == ug.ntile - 1;
+                    const int nwidth = nlast ? (last ? ng.last_width : ug.last_width) : kColTile;
+                    const int vbuf = g.s;
+                    const uint32_t vphase = g.phase;
                     g.next(P.stages);
-                    SA_TR(r, 30);
-                    // S of the next tile, which may be the next unit's first
-                    if (!last) {
-                        const bool nlast = t + 1 == ug.ntile - 1;
-                        issue_s(nlast, nlast ? ug.last_width : kColTile);
-                    } else {
-                        w.next(P);
-                        ++nu;
-                        if (w.valid(P)) {
-                            const UnitGeom ng = w.geom(P);
-                            mbar_wait<kAReady>(rb, nu & 1, wctx, 4);
-                            issue_s(ng.ntile == 1, ng.ntile == 1 ? ng.last_width : kColTile);
+                    const int kbuf = g.s;
+                    const uint32_t kphase = g.phase;
+                    g.next(P.stages);
+                    const uint32_t idesc = make_idesc(128, HD, false, true, F16);
+                    const uint32_t db = desc_lo(smem_base + L::kRing + vbuf * L::kStageBytes, L::kStageSlab);
+#pragma unroll 1
+                    for (int r = 0; r < nrt; ++r) {
+                        const uint32_t rb = smem_base + r * 8;
+                        const uint32_t tm_s = tmem_base + r * kColTile, tm_t = tmem_t0 + r * HD;
+                        mbar_wait<kFull>(smem_base + vbuf * 8, vphase, wctx, 6);
+                        SA_TR(0, 41 + 100 * r);
+                        // the previous unit's T has been read out by the auxiliary group
+                        if (t == 0 && nu > 0) mbar_wait<kTFree>(rb, (nu - 1) & 1, wctx, 10);
+                        mbar_wait<kPReady>(rb, n & 1, wctx, 5);
+                        SA_TR(0, 20 + 100 * r);
+                        tc_fence_after();
+                        static_for<8>([&](auto kk_c) {
+                            constexpr int kk = decltype(kk_c)::value;
+                            if (kk < ksteps) mma_ts_lo<kk * 8, kk * (2048 >> 4)>(leader, tm_t, tm_s, db, idesc, t > 0 || kk > 0);
+                        });
+                        SA_TR(0, 29 + 100 * r);
+                        tc_commit<kEmpty>(leader, smem_base + vbuf * 8);
+                        if (last) tc_commit<kOReady>(leader, rb);
+                        SA_TR(0, 30 + 100 * r);
+                        if (have_next) {
+                            mbar_wait<kFull>(smem_base + kbuf * 8, kphase, wctx, 3);
+                            SA_TR(0, 31 + 100 * r);
+                            if (last) mbar_wait<kAReady>(rb, (nu + 1) & 1, wctx, 4);
+                            tc_fence_after();
+                            issue_s(r, kbuf, nlast, nwidth);
                         }
+                        SA_TR(0, 40 + 100 * r);
                     }
-                    SA_TR(r, 40);
                 }
-                if (w.valid(P)) ug = w.geom(P);
+                w = wn;
+                ug = ng;
+                ++nu;
             }
         }
     } else if (warp >= 8) {
@@ -636,15 +656,14 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                 SA_TR(4 + r, 70);
                 tc_fence_after();
                 // One column tile of up to NC columns.  The scores are read twice, once for the maximum and once, 16 columns
-                // ahead, for the exponentials: keeping 64 of them in registers spilled even at 128 registers.  The P.V MMAs
-                // of the first 64 columns start under the exponentials of the rest.
+                // ahead, for the exponentials: keeping 64 of them in registers spilled even at 128 registers.
                 auto softmax = [&](auto nc_c, auto masked_c) {
                     constexpr int NC = decltype(nc_c)::value;
                     constexpr bool MASKED = decltype(masked_c)::value;
                     // masked scores (whatever the buffer holds there) become -inf
                     auto mask = [&](auto& x, int c0, auto n_c) {
-                        constexpr int N = decltype(n_c)::value;
                         if constexpr (MASKED) {
+                            constexpr int N = decltype(n_c)::value;
                             const int a = max(lo - c0, 0), z = min(hi - c0, N - 1);
                             const uint32_t bits = z >= a ? (~0u >> (31 - (z - a))) << a : 0u;
 #pragma unroll
@@ -710,13 +729,10 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                             pk[e >> 1] = E::pack(pe.x, pe.y);
                         }
                         tmem_st8(s_addr + 8 * c, pk);
-                        if (c == 3 || c == NC / 16 - 1) {
-                            tmem_wait_st();
-                            tc_fence_before();
-                            if (c == 3 || NC < 64) SA_FWD_ARRIVE(kP0Ready, rb);
-                        }
                     }
-                    SA_FWD_ARRIVE(kP1Ready, rb);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    SA_FWD_ARRIVE(kPReady, rb);
                     l += ls.x + ls.y;
                 };
                 // a tile is "full" when every column is inside every row's window: no masks needed
