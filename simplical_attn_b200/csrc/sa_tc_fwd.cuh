@@ -137,7 +137,10 @@ struct UnitWalk {
         const int qpb = (P.row_tiles * kRowTile) >> P.dw_log2;
         g.i0 = qb * qpb;
         const int i_last = min(g.i0 + qpb, p.N) - 1;
-        g.col_start = max(0, g.i0 + p.halo1 - p.w1 + 1);
+        // (the pair's first query also where row tiles are single: a query's column tiles, and with them the rounding of
+        // its result, do not depend on how many heads the call holds)
+        const int i_pair = g.i0 & ~(((kNumRowTiles * kRowTile) >> P.dw_log2) - 1);
+        g.col_start = max(0, i_pair + p.halo1 - p.w1 + 1);
         const int ncols = i_last + p.halo1 - g.col_start + 1;
         g.ntile = (ncols + kColTile - 1) / kColTile;
         g.last_width = ((ncols - (g.ntile - 1) * kColTile) + 15) & ~15;
