@@ -555,7 +555,7 @@ int sa_forward_status(const sa_params* p, const void* q, const void* k1, const v
         algo = SA_ALGO_GENERAL;
     }
     if (algo == SA_ALGO_TCGEN05) return launch_fwd_tc(p, k, q, k1, k2, v1, v2, o, lse, workspace, status, st);
-    const cudaError_t e = sa::general::launch_fwd(p->dtype, k, q, k1, k2, v1, v2, o, lse, st);
+    const cudaError_t e = sa::general::launch_fwd(p->dtype, k, q, k1, k2, v1, v2, o, lse, device_info().sm_count, st);
     g_launches += 1;
     return e == cudaSuccess ? SA_OK : SA_ERR_LAUNCH;
 }
@@ -595,7 +595,8 @@ int sa_backward_status(const sa_params* p, const void* q, const void* k1, const 
         if (rc != -1) return rc;      // -1: the tensor-core backward declines this problem
         if (p->algo == SA_ALGO_TCGEN05) return SA_ERR_UNSUPPORTED;
     }
-    const cudaError_t e = sa::general::launch_bwd(p->dtype, k, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, st);
+    const cudaError_t e =
+        sa::general::launch_bwd(p->dtype, k, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, device_info().sm_count, st);
     g_launches += (dq ? 1 : 0) + ((dk1 || dv1) ? 1 : 0) + ((dk2 || dv2) ? 1 : 0);
     return e == cudaSuccess ? SA_OK : SA_ERR_LAUNCH;
 }

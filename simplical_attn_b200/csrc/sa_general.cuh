@@ -1,332 +1,699 @@
 // General 2-simplicial attention kernels: CUDA-core fp32 arithmetic for any dtype, head dim
-// (<= 256) and window.  One warp owns one output row and accumulates it in registers, so every
-// output element is written exactly once, in a fixed order, without atomics.
+// (<= 256) and window.  Every output element is written exactly once, in a fixed order, without atomics.
 //
-// They cover what the tensor-core kernels do not (fp16/fp32 tensors, head dims other than 64/128,
+// They cover what the tensor-core kernels do not (fp32 tensors, head dims other than 64/128, unaligned rows,
 // very wide K2 windows) and are the on-device cross-check of the tensor-core kernels.
 //
 // The arithmetic restates the reference's definition (simplicial/reference.py:39-74) with an
 // online maximum, and, for the backward, the derivative the reference's backward kernels
 // implement (simplicial/kernels.py:175-382 for dQ/dK1/dV1, :386-566 for dK2/dV2).
+//
+// A block works on tiles of 64 virtual rows (query i, K2 row k) with operand rows A = Q_i * (K2_k + bias) * scale and
+// C = dO_i * (V2_k + bias) against tiles of K1/V1 rows, all in shared memory as fp32; a thread holds 4 rows by up to 4
+// columns of the score tile and 4 rows by D/16 columns of the accumulators, so an operand read from shared memory is
+// used four times.  Large problems are bound by the FMA pipes and shared-memory reads at about equal shares, small ones
+// by the latency of a block's chain of loads.  (One warp per output row with the head dim across its lanes, as
+// before, spent five to ten shuffles in a serial chain on every (j, k) pair: all kernels of a forward and backward
+// together 846 -> 141 us for fp32 B1 N256 H2 D64 w 64/16, 1448 -> 463 us for bf16 B2 N512 H4 D32 w 32/32.)
 #pragma once
+
+#include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "sa_common.cuh"
 
 namespace sa {
 namespace general {
 
-constexpr int kWarpsPerBlock = 4;
+constexpr int kThreads = 256;        // 16 x 16
+constexpr int kRows = 64;            // virtual rows of a tile
+constexpr int kMaxOwners = 16;       // queries (K2 rows) whose virtual rows a tile holds, at most
+constexpr int kColRows = 32;         // K1/V1 rows a block of the dK1/dV1 kernel owns
 
-// Lane `lane` of a warp holds elements d = lane + 32*e of a D-vector.
-template <typename T, int EPL>
-__device__ __forceinline__ void load_row(const T* __restrict__ row, int D, int lane, float (&v)[EPL], float bias = 0.f) {
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-        const int d = lane + 32 * e;
-        v[e] = d < D ? to_f<T>(row[d]) + bias : 0.f;
+// Shared memory for head dims up to DP: row pitch DP + 4 floats, so that 16-byte reads of consecutive rows fall into
+// different banks.
+template <int DP>
+struct Shape {
+    static constexpr int kCols = DP <= 128 ? 64 : 32;       // K1/V1 rows of a tile
+    static constexpr int kPitch = DP + 4;
+    static constexpr int kPPitch = kCols + 4;
+    static constexpr int kUnroll = DP <= 128 ? 16 : 8;      // global loads in flight per thread
+    static constexpr int kDpt = DP / 16;                    // accumulator columns per thread and row
+    static constexpr int kVec = kDpt < 4 ? kDpt : 4;        // ... in groups of kVec consecutive ones, 16 kVec apart
+    static constexpr int kRowTile = kRows * kPitch;         // floats
+    static constexpr int kColTile = kCols * kPitch;
+    static constexpr int kPTile = kRows * kPPitch;
+    static constexpr int kStats = 8 * kRows + 4 * kMaxOwners;
+    static constexpr int kFwdBytes = (kRowTile + 2 * kColTile + kPTile + kStats) * 4;
+    static constexpr int kBwdBytes = (2 * kRowTile + 2 * kColTile + 2 * kPTile + kStats) * 4;
+    static constexpr int kColPPitch = kColRows + 4;
+    static constexpr int kColBytes = (2 * kRowTile + 2 * kColRows * kPitch + 2 * kRows * kColPPitch + kStats) * 4;
+    static_assert(kBwdBytes <= 227 * 1024 && kColBytes <= 227 * 1024, "shared memory of a block");
+};
+
+__device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) < INFINITY); }
+
+template <int N>
+__device__ __forceinline__ void lds_vec(const float* p, float (&v)[N]) {
+    if constexpr (N == 4) {
+        const float4 t = *(const float4*)p;
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+        const float2 t = *(const float2*)p;
+        v[0] = t.x; v[1] = t.y;
     }
 }
 
-template <typename T, int EPL>
-__device__ __forceinline__ void store_row(T* __restrict__ row, int D, int lane, const float (&v)[EPL]) {
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-        const int d = lane + 32 * e;
-        if (d < D) row[d] = from_f<T>(v[e]);
+// Rows [r0, r0 + count) of x (row stride xs) -> dst, fp32, zeros behind `avail` rows and behind D.  True if a value is
+// not finite.
+template <typename T, int DP>
+__device__ __forceinline__ bool load_rows(float* dst, const T* __restrict__ x, int64_t xs, int r0, int count, int avail, int D) {
+    bool bad = false;
+#pragma unroll Shape<DP>::kUnroll
+    for (int idx = threadIdx.x; idx < count * DP; idx += kThreads) {
+        const int r = idx / DP, d = idx % DP;
+        const float v = r < avail && d < D ? to_f<T>(x[(int64_t)(r0 + r) * xs + d]) : 0.f;
+        bad |= not_finite(v);
+        dst[r * Shape<DP>::kPitch + d] = v;
+    }
+    return bad;
+}
+
+// The operand rows of a tile: dst[r] = x[ri[r]] * (y[rk[r]] + bias) * mult, zeros where ri[r] < 0.
+template <typename T, int DP>
+__device__ __forceinline__ void form_rows(float* dst, const int* ri, const int* rk, const T* __restrict__ x, int64_t xs,
+                                          const T* __restrict__ y, int64_t ys, float bias, float mult, int D) {
+#pragma unroll Shape<DP>::kUnroll
+    for (int idx = threadIdx.x; idx < kRows * DP; idx += kThreads) {
+        const int r = idx / DP, d = idx % DP;
+        float v = 0.f;
+        if (ri[r] >= 0 && d < D) v = to_f<T>(x[(int64_t)ri[r] * xs + d]) * (to_f<T>(y[(int64_t)rk[r] * ys + d]) + bias) * mult;
+        dst[r * Shape<DP>::kPitch + d] = v;
     }
 }
 
-template <int EPL>
-__device__ __forceinline__ float dot(const float (&a)[EPL], const float (&b)[EPL]) {
+// Delta = dO . O and LSE of every row of a tile, four threads to a row.  head_of(r, 0 | 1 | 2): offset of the row's
+// head in o, d_o and lse.
+template <typename T, typename F>
+__device__ __forceinline__ void row_stats(float* delta, float* L, const int* ri, const T* __restrict__ o, int64_t os,
+                                          const T* __restrict__ d_o, int64_t dos, const float* __restrict__ lse, int D, F head_of) {
+    const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
     float s = 0.f;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) s = fmaf(a[e], b[e], s);
-    return s;
+    const int i = ri[r];
+    if (i >= 0) {
+        const T* orow = o + head_of(r, 0) + (int64_t)i * os;
+        const T* drow = d_o + head_of(r, 1) + (int64_t)i * dos;
+#pragma unroll 8
+        for (int d = part; d < D; d += 4) s = fmaf(to_f<T>(drow[d]), to_f<T>(orow[d]), s);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (part == 0) {
+        delta[r] = s;
+        L[r] = i >= 0 ? lse[head_of(r, 2) + i] : 0.f;
+    }
 }
 
-// Forward: warp per (b, h, i).
-template <typename T, int EPL>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-fwd_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2,
+// s[a][c] = X[4 ty + a] . Y[tx + 16 c]
+template <int DP, int NC>
+__device__ __forceinline__ void product(const float* X, const float* Y, int ty, int tx, float (&s)[4][NC]) {
+    constexpr int P = Shape<DP>::kPitch;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[a][c] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < DP; d += 4) {
+        float x[4][4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) lds_vec<4>(X + (4 * ty + a) * P + d, x[a]);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            float y[4];
+            lds_vec<4>(Y + (tx + 16 * c) * P + d, y);
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[a][c] = fmaf(x[a][e], y[e], s[a][c]);
+        }
+    }
+}
+
+// acc[a][.] += sum over j < n of W[4 ty + a][j] Y[j][.].  CHECK: Y holds values that are not finite; a row that does not
+// see column j (W = 0 there) must not meet them.
+template <int DP, bool CHECK>
+__device__ __forceinline__ void accumulate(float (&acc)[4][Shape<DP>::kDpt], const float* W, const float* Y, int n, int ty, int tx,
+                                           const int (&lo)[4], const int (&hi)[4]) {
+    using S = Shape<DP>;
+    constexpr int V = S::kVec, NV = S::kDpt / V;
+#pragma unroll 2
+    for (int j = 0; j < n; j += 4) {
+        float w[4][4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) lds_vec<4>(W + (4 * ty + a) * S::kPPitch + j, w[a]);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                float y[V];
+                lds_vec<V>(Y + (j + jj) * S::kPitch + tx * V + 16 * V * v, y);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    if (CHECK && (j + jj < lo[a] || j + jj > hi[a])) continue;
+#pragma unroll
+                    for (int e = 0; e < V; ++e) acc[a][V * v + e] = fmaf(w[a][jj], y[e], acc[a][V * v + e]);
+                }
+            }
+    }
+}
+
+// W[4 ty + a][.] = acc * (x[idx[row]] + bias) * mult, zeros where ri < 0.
+template <typename T, int DP>
+__device__ __forceinline__ void scale_out(float* W, const float (&acc)[4][Shape<DP>::kDpt], const int* ri, const int* idx,
+                                          const T* __restrict__ x, int64_t xs, float bias, float mult, int D, int ty, int tx) {
+    using S = Shape<DP>;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int r = 4 * ty + a;
+#pragma unroll
+        for (int e = 0; e < S::kDpt; ++e) {
+            const int d = (e / S::kVec) * 16 * S::kVec + tx * S::kVec + e % S::kVec;
+            W[r * S::kPitch + d] = ri[r] >= 0 && d < D ? acc[a][e] * ((to_f<T>(x[(int64_t)idx[r] * xs + d]) + bias) * mult) : 0.f;
+        }
+    }
+}
+
+// Calls f with the number of 16-column groups that hold n columns.
+template <int MAX, typename F>
+__device__ __forceinline__ void with_groups(int n, F&& f) {
+    if constexpr (MAX == 1) {
+        f(std::integral_constant<int, 1>{});
+    } else {
+        if (n > 16 * (MAX - 1)) f(std::integral_constant<int, MAX>{});
+        else with_groups<MAX - 1>(n, static_cast<F&&>(f));
+    }
+}
+
+// Columns of the K1/V1 row tile at j0 that query i sees, relative to j0.
+__device__ __forceinline__ void window(const KParams& p, int i, int j0, int& lo, int& hi) {
+    hi = i < 0 ? -1 : i + p.halo1 - j0;
+    lo = i < 0 ? 0 : max(0, i + p.halo1 - p.w1 + 1) - j0;
+}
+
+// Forward.  A block owns `owners` consecutive queries of one head (as many as fit 64 rows of w2 each; one, in several
+// passes over 64 K2 rows, where w2 > 64).
+template <typename T, int DP>
+__global__ void __launch_bounds__(kThreads)
+fwd_kernel(KParams p, int owners, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2,
            const T* __restrict__ v1, const T* __restrict__ v2, T* __restrict__ o, float* __restrict__ lse) {
-    const long row = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= (long)p.B * p.H * p.N) return;
-    const int i = (int)(row % p.N);
-    const int h = (int)((row / p.N) % p.H);
-    const int b = (int)(row / p.N / p.H);
+    using S = Shape<DP>;
+    extern __shared__ __align__(16) float sm[];
+    float *As = sm, *Ks = As + S::kRowTile, *Vs = Ks + S::kColTile, *Ps = Vs + S::kColTile, *st = Ps + S::kPTile;
+    int *ri = (int*)st, *rk = ri + kRows;
+    float *row_m = st + 2 * kRows, *row_l = row_m + kRows, *own_m = row_l + kRows, *own_l = own_m + kMaxOwners, *own_f = own_l + kMaxOwners;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int nblk = (p.N + owners - 1) / owners;
+    const int i0 = (int)(blockIdx.x % nblk) * owners, h = (int)(blockIdx.x / nblk % p.H), b = (int)(blockIdx.x / nblk / p.H);
     const int hk = h / p.G;
-    const int D = p.D;
-
-    float qv[EPL];
-    load_row<T, EPL>(q + b * p.q.b + (long)i * p.q.n + h * p.q.h, D, lane, qv);
-    const int j_hi = i + p.halo1, j_lo = max(0, j_hi - p.w1 + 1);
-    const int k_hi = i + p.halo2, k_lo = max(0, k_hi - p.w2 + 1);
+    const T* qh = q + b * p.q.b + h * p.q.h;
     const T* k1h = k1 + b * p.k1.b + hk * p.k1.h;
     const T* v1h = v1 + b * p.v1.b + hk * p.v1.h;
     const T* k2h = k2 + b * p.k2.b + hk * p.k2.h;
     const T* v2h = v2 + b * p.v2.b + hk * p.v2.h;
-
-    float m = -INFINITY, l = 0.f;
-    float acc[EPL];
+    const int per = min(p.w2, kRows);                   // rows of one owner in a tile
+    const int i_last = min(i0 + owners, p.N) - 1;
+    const int j_lo = max(0, i0 + p.halo1 - p.w1 + 1), j_hi = i_last + p.halo1;
+    float out[DP / 16];                                 // sum over K2 rows, element tid + 256 x of [owners][DP]
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
-
-    for (int k = k_lo; k <= k_hi; ++k) {
-        float a[EPL], t[EPL], v2v[EPL];
-        load_row<T, EPL>(k2h + (long)k * p.k2.n, D, lane, a, p.k2_bias);
-        load_row<T, EPL>(v2h + (long)k * p.v2.n, D, lane, v2v, p.v2_bias);
+    for (int x = 0; x < DP / 16; ++x) out[x] = 0.f;
+    if (tid < kMaxOwners) { own_m[tid] = -INFINITY; own_l[tid] = 0.f; }
+    for (int d0 = 0; d0 < p.w2; d0 += kRows) {
+        __syncthreads();
+        if (tid < kRows) {
+            const int own = tid / per, dlt = d0 + tid % per, i = i0 + own, kb = i + p.halo2 - dlt;
+            const bool ok = own < owners && i < p.N && dlt < p.w2 && kb >= 0;
+            ri[tid] = ok ? i : -1;
+            rk[tid] = kb;
+        }
+        __syncthreads();
+        form_rows<T, DP>(As, ri, rk, qh, p.q.n, k2h, p.k2.n, p.k2_bias, p.scale, p.D);
+        float m[4], l[4], t[4][S::kDpt];
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) { a[e] *= qv[e] * p.scale; t[e] = 0.f; }
-        for (int j = j_lo; j <= j_hi; ++j) {
-            float k1v[EPL], v1v[EPL];
-            load_row<T, EPL>(k1h + (long)j * p.k1.n, D, lane, k1v);
-            load_row<T, EPL>(v1h + (long)j * p.v1.n, D, lane, v1v);
-            const float s = warp_sum(dot<EPL>(a, k1v));
-            if (s > m) {                                  // warp-uniform
-                const float corr = __expf(m - s);         // m = -inf gives 0
-                l *= corr;
+        for (int a = 0; a < 4; ++a) {
+            m[a] = -INFINITY;
+            l[a] = 0.f;
 #pragma unroll
-                for (int e = 0; e < EPL; ++e) { acc[e] *= corr; t[e] *= corr; }
-                m = s;
-            }
-            const float pv = __expf(s - m);
-            l += pv;
+            for (int e = 0; e < S::kDpt; ++e) t[a][e] = 0.f;
+        }
+        for (int j0 = j_lo; j0 <= j_hi; j0 += S::kCols) {
+            const int n = min(j_hi - j0 + 1, S::kCols);
+            const int n16 = (n + 15) & ~15;             // columns computed
+            __syncthreads();
+            load_rows<T, DP>(Ks, k1h, p.k1.n, j0, n16, n, p.D);
+            const bool bad = load_rows<T, DP>(Vs, v1h, p.v1.n, j0, n16, n, p.D);
+            const bool check = __syncthreads_or(bad);
+            int lo[4], hi[4];
 #pragma unroll
-            for (int e = 0; e < EPL; ++e) t[e] = fmaf(pv, v1v[e], t[e]);
+            for (int a = 0; a < 4; ++a) window(p, ri[4 * ty + a], j0, lo[a], hi[a]);
+            with_groups<S::kCols / 16>(n, [&](auto nc) {
+                constexpr int NC = decltype(nc)::value;
+                float s[4][NC];
+                product<DP, NC>(As, Ks, ty, tx, s);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    float mx = m[a];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (tx + 16 * c >= lo[a] && tx + 16 * c <= hi[a]) mx = fmaxf(mx, s[a][c]);
+#pragma unroll
+                    for (int x = 8; x >= 1; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+                    const float corr = mx == m[a] ? 1.f : __expf(m[a] - mx);      // m = -inf gives 0
+                    m[a] = mx;
+                    l[a] *= corr;
+#pragma unroll
+                    for (int e = 0; e < S::kDpt; ++e) t[a][e] *= corr;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const float pv = tx + 16 * c >= lo[a] && tx + 16 * c <= hi[a] ? __expf(s[a][c] - mx) : 0.f;
+                        l[a] += pv;
+                        Ps[(4 * ty + a) * S::kPPitch + tx + 16 * c] = pv;
+                    }
+                }
+            });
+            __syncwarp();                               // a warp reads back the rows it wrote
+            if (check) accumulate<DP, true>(t, Ps, Vs, n16, ty, tx, lo, hi);
+            else accumulate<DP, false>(t, Ps, Vs, n16, ty, tx, lo, hi);
         }
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) acc[e] = fmaf(t[e], v2v[e], acc[e]);
-    }
-    const float inv = 1.f / l;
+        for (int a = 0; a < 4; ++a) {
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) acc[e] *= inv;
-    store_row<T, EPL>(o + b * p.o.b + (long)i * p.o.n + h * p.o.h, D, lane, acc);
-    if (lane == 0) lse[((long)b * p.H + h) * p.N + i] = m + logf(l);
+            for (int x = 8; x >= 1; x >>= 1) l[a] += __shfl_xor_sync(0xffffffffu, l[a], x);
+            if (tx == 0) {
+                row_m[4 * ty + a] = m[a];
+                row_l[4 * ty + a] = l[a];
+            }
+        }
+        __syncthreads();                                // (A is no longer read)
+        float* W = As;
+        scale_out<T, DP>(W, t, ri, rk, v2h, p.v2.n, p.v2_bias, 1.f, p.D, ty, tx);
+        if (tid < owners) {
+            float mq = own_m[tid], lq = own_l[tid];
+            for (int r = tid * per; r < (tid + 1) * per; ++r)
+                if (ri[r] >= 0) mq = fmaxf(mq, row_m[r]);
+            const float f = own_m[tid] == mq ? 1.f : __expf(own_m[tid] - mq);      // -inf gives 0
+            lq *= f;
+            for (int r = tid * per; r < (tid + 1) * per; ++r) {
+                const float e = ri[r] >= 0 ? __expf(row_m[r] - mq) : 0.f;
+                lq += e * row_l[r];
+                row_m[r] = e;                           // from here on the row's weight
+            }
+            own_m[tid] = mq;
+            own_l[tid] = lq;
+            own_f[tid] = f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int x = 0; x < DP / 16; ++x) {
+            const int own = (tid + kThreads * x) / DP, d = (tid + kThreads * x) % DP;
+            if (own < owners) {
+                float a = out[x] * own_f[own];
+                for (int r = own * per; r < (own + 1) * per; ++r)
+                    if (ri[r] >= 0) a = fmaf(row_m[r], W[r * S::kPitch + d], a);
+                out[x] = a;
+            }
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < DP / 16; ++x) {
+        const int own = (tid + kThreads * x) / DP, d = (tid + kThreads * x) % DP;
+        if (own < owners && i0 + own < p.N && d < p.D)
+            o[b * p.o.b + (int64_t)(i0 + own) * p.o.n + h * p.o.h + d] = from_f<T>(out[x] * (1.f / own_l[own]));
+    }
+    if (tid < owners && i0 + tid < p.N) lse[((long)b * p.H + h) * p.N + i0 + tid] = own_m[tid] + logf(own_l[tid]);
 }
 
-// Per-query quantities every backward sweep needs: the query row, dO row, Delta = dO.O and LSE.
-template <typename T, int EPL>
-__device__ __forceinline__ void load_query(const KParams& p, const T* q, const T* o, const T* d_o, const float* lse,
-                                           int b, int h, int i, int lane, float (&qv)[EPL], float (&dov)[EPL],
-                                           float& delta, float& L) {
-    float ov[EPL];
-    load_row<T, EPL>(q + b * p.q.b + (long)i * p.q.n + h * p.q.h, p.D, lane, qv);
-    load_row<T, EPL>(d_o + b * p.d_o.b + (long)i * p.d_o.n + h * p.d_o.h, p.D, lane, dov);
-    load_row<T, EPL>(o + b * p.o.b + (long)i * p.o.n + h * p.o.h, p.D, lane, ov);
-    delta = warp_sum(dot<EPL>(dov, ov));
-    L = lse[((long)b * p.H + h) * p.N + i];
-}
-
-// dQ: warp per (b, h, i).
-template <typename T, int EPL>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-bwd_dq_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2,
-              const T* __restrict__ v1, const T* __restrict__ v2, const T* __restrict__ o,
-              const float* __restrict__ lse, const T* __restrict__ d_o, T* __restrict__ dq) {
-    const long row = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= (long)p.B * p.H * p.N) return;
-    const int i = (int)(row % p.N);
-    const int h = (int)((row / p.N) % p.H);
-    const int b = (int)(row / p.N / p.H);
-    const int hk = h / p.G;
-    const int D = p.D;
-    float qv[EPL], dov[EPL], delta, L;
-    load_query<T, EPL>(p, q, o, d_o, lse, b, h, i, lane, qv, dov, delta, L);
-    const int j_hi = i + p.halo1, j_lo = max(0, j_hi - p.w1 + 1);
-    const int k_hi = i + p.halo2, k_lo = max(0, k_hi - p.w2 + 1);
+// dQ (KV2 = false): a block owns `owners` queries of one head.  dK2 and dV2 (KV2 = true): `owners` K2 rows of one KV
+// head, summed over the group's query heads.  Tiles as in the forward.
+template <typename T, int DP, bool KV2>
+__global__ void __launch_bounds__(kThreads)
+bwd_row_kernel(KParams p, int owners, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2,
+               const T* __restrict__ v1, const T* __restrict__ v2, const T* __restrict__ o, const float* __restrict__ lse,
+               const T* __restrict__ d_o, T* __restrict__ dq, T* __restrict__ dk2, T* __restrict__ dv2) {
+    using S = Shape<DP>;
+    extern __shared__ __align__(16) float sm[];
+    float *As = sm, *Cs = As + S::kRowTile, *Ks = Cs + S::kRowTile, *Vs = Ks + S::kColTile;
+    float *Ps = Vs + S::kColTile, *Ds = Ps + S::kPTile, *st = Ds + S::kPTile;
+    int *ri = (int*)st, *rk = ri + kRows;
+    float *delta = st + 2 * kRows, *L = delta + kRows;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int n_own = KV2 ? p.n2 : p.N, heads = KV2 ? p.Hkv : p.H;
+    const int nblk = (n_own + owners - 1) / owners;
+    const int x0 = (int)(blockIdx.x % nblk) * owners, hb = (int)(blockIdx.x / nblk % heads), b = (int)(blockIdx.x / nblk / heads);
+    const int hk = KV2 ? hb : hb / p.G;
     const T* k1h = k1 + b * p.k1.b + hk * p.k1.h;
     const T* v1h = v1 + b * p.v1.b + hk * p.v1.h;
     const T* k2h = k2 + b * p.k2.b + hk * p.k2.h;
     const T* v2h = v2 + b * p.v2.b + hk * p.v2.h;
-    float acc[EPL];
+    const int per = min(p.w2, kRows);
+    float outg[DP / 16], outu[KV2 ? DP / 16 : 1];
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
-    for (int k = k_lo; k <= k_hi; ++k) {
-        float k2v[EPL], a[EPL], c[EPL], g[EPL];
-        load_row<T, EPL>(k2h + (long)k * p.k2.n, D, lane, k2v, p.k2_bias);
-        load_row<T, EPL>(v2h + (long)k * p.v2.n, D, lane, c, p.v2_bias);
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) { a[e] = qv[e] * k2v[e] * p.scale; c[e] *= dov[e]; g[e] = 0.f; }
-        for (int j = j_lo; j <= j_hi; ++j) {
-            float k1v[EPL], v1v[EPL];
-            load_row<T, EPL>(k1h + (long)j * p.k1.n, D, lane, k1v);
-            load_row<T, EPL>(v1h + (long)j * p.v1.n, D, lane, v1v);
-            const float s = warp_sum(dot<EPL>(a, k1v));
-            const float dP = warp_sum(dot<EPL>(c, v1v));
-            const float dS = __expf(s - L) * (dP - delta);
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) g[e] = fmaf(dS, k1v[e], g[e]);
-        }
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) acc[e] = fmaf(g[e], k2v[e] * p.scale, acc[e]);
+    for (int x = 0; x < DP / 16; ++x) {
+        outg[x] = 0.f;
+        if (KV2) outu[x] = 0.f;
     }
-    store_row<T, EPL>(dq + b * p.dq.b + (long)i * p.dq.n + h * p.dq.h, D, lane, acc);
+    for (int hq = 0; hq < (KV2 ? p.G : 1); ++hq) {
+        const int h = KV2 ? hk * p.G + hq : hb;
+        const T* qh = q + b * p.q.b + h * p.q.h;
+        const T* doh = d_o + b * p.d_o.b + h * p.d_o.h;
+        for (int d0 = 0; d0 < p.w2; d0 += kRows) {
+            // queries of the tile's rows
+            const int d1 = min(d0 + kRows, p.w2) - 1;
+            const int i_lo = KV2 ? max(0, x0 - p.halo2 + d0) : x0;
+            const int i_hi = min(p.N - 1, KV2 ? min(x0 + owners, n_own) - 1 - p.halo2 + d1 : x0 + owners - 1);
+            if (i_hi < i_lo) continue;                  // (the same for the whole block)
+            __syncthreads();
+            if (tid < kRows) {
+                const int own = tid / per, dlt = d0 + tid % per;
+                const int kb = KV2 ? x0 + own : x0 + own + p.halo2 - dlt, i = KV2 ? kb - p.halo2 + dlt : x0 + own;
+                const bool ok = own < owners && i >= 0 && i < p.N && dlt < p.w2 && kb >= 0 && kb < p.n2;
+                ri[tid] = ok ? i : -1;
+                rk[tid] = kb;
+            }
+            __syncthreads();
+            form_rows<T, DP>(As, ri, rk, qh, p.q.n, k2h, p.k2.n, p.k2_bias, p.scale, p.D);
+            form_rows<T, DP>(Cs, ri, rk, doh, p.d_o.n, v2h, p.v2.n, p.v2_bias, 1.f, p.D);
+            row_stats<T>(delta, L, ri, o, p.o.n, d_o, p.d_o.n, lse, p.D, [&](int, int what) -> int64_t {
+                return what == 0 ? b * p.o.b + h * p.o.h : what == 1 ? b * p.d_o.b + h * p.d_o.h : ((int64_t)b * p.H + h) * p.N;
+            });
+            float g[4][S::kDpt], u[KV2 ? 4 : 1][S::kDpt];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int e = 0; e < S::kDpt; ++e) {
+                    g[a][e] = 0.f;
+                    if (KV2) u[a][e] = 0.f;
+                }
+            const int j_lo = max(0, i_lo + p.halo1 - p.w1 + 1), j_hi = i_hi + p.halo1;
+            for (int j0 = j_lo; j0 <= j_hi; j0 += S::kCols) {
+                const int n = min(j_hi - j0 + 1, S::kCols);
+                const int n16 = (n + 15) & ~15;
+                __syncthreads();
+                bool bad = load_rows<T, DP>(Ks, k1h, p.k1.n, j0, n16, n, p.D);
+                bad |= load_rows<T, DP>(Vs, v1h, p.v1.n, j0, n16, n, p.D);
+                const bool check = __syncthreads_or(bad);
+                int lo[4], hi[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) window(p, ri[4 * ty + a], j0, lo[a], hi[a]);
+                with_groups<S::kCols / 16>(n, [&](auto nc) {
+                    constexpr int NC = decltype(nc)::value;
+                    float s[4][NC], dp[4][NC];
+                    product<DP, NC>(As, Ks, ty, tx, s);
+                    product<DP, NC>(Cs, Vs, ty, tx, dp);
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        const float la = L[4 * ty + a], de = delta[4 * ty + a];
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            const bool ok = tx + 16 * c >= lo[a] && tx + 16 * c <= hi[a];
+                            const float pv = ok ? __expf(s[a][c] - la) : 0.f;
+                            if (KV2) Ps[(4 * ty + a) * S::kPPitch + tx + 16 * c] = pv;
+                            Ds[(4 * ty + a) * S::kPPitch + tx + 16 * c] = ok ? pv * (dp[a][c] - de) : 0.f;
+                        }
+                    }
+                });
+                __syncwarp();                           // a warp reads back the rows it wrote
+                if (check) accumulate<DP, true>(g, Ds, Ks, n16, ty, tx, lo, hi);
+                else accumulate<DP, false>(g, Ds, Ks, n16, ty, tx, lo, hi);
+                if constexpr (KV2) {
+                    if (check) accumulate<DP, true>(u, Ps, Vs, n16, ty, tx, lo, hi);
+                    else accumulate<DP, false>(u, Ps, Vs, n16, ty, tx, lo, hi);
+                }
+            }
+            __syncthreads();                            // (A and C are no longer read)
+            if constexpr (KV2) {
+                scale_out<T, DP>(As, g, ri, ri, qh, p.q.n, 0.f, p.scale, p.D, ty, tx);
+                scale_out<T, DP>(Cs, u, ri, ri, doh, p.d_o.n, 0.f, 1.f, p.D, ty, tx);
+            } else {
+                scale_out<T, DP>(As, g, ri, rk, k2h, p.k2.n, p.k2_bias, p.scale, p.D, ty, tx);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int x = 0; x < DP / 16; ++x) {
+                const int own = (tid + kThreads * x) / DP, d = (tid + kThreads * x) % DP;
+                if (own < owners)
+                    for (int r = own * per; r < (own + 1) * per; ++r) {
+                        outg[x] += As[r * S::kPitch + d];
+                        if (KV2) outu[x] += Cs[r * S::kPitch + d];
+                    }
+            }
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < DP / 16; ++x) {
+        const int own = (tid + kThreads * x) / DP, d = (tid + kThreads * x) % DP, r = x0 + own;
+        if (own < owners && r < n_own && d < p.D) {
+            if constexpr (KV2) {
+                if (dk2) dk2[b * p.dk2.b + (int64_t)r * p.dk2.n + hb * p.dk2.h + d] = from_f<T>(outg[x]);
+                if (dv2) dv2[b * p.dv2.b + (int64_t)r * p.dv2.n + hb * p.dv2.h + d] = from_f<T>(outu[x]);
+            } else {
+                dq[b * p.dq.b + (int64_t)r * p.dq.n + hb * p.dq.h + d] = from_f<T>(outg[x]);
+            }
+        }
+    }
 }
 
-// dK1 and dV1: warp per (b, hkv, K1 buffer row); loops over the group's query heads.
-template <typename T, int EPL>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-bwd_kv1_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2,
-               const T* __restrict__ v1, const T* __restrict__ v2, const T* __restrict__ o,
-               const float* __restrict__ lse, const T* __restrict__ d_o, T* __restrict__ dk1, T* __restrict__ dv1) {
-    const long row = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= (long)p.B * p.Hkv * p.n1) return;
-    const int jb = (int)(row % p.n1);
-    const int hk = (int)((row / p.n1) % p.Hkv);
-    const int b = (int)(row / p.n1 / p.Hkv);
-    const int D = p.D;
-    float k1v[EPL], v1v[EPL], acck[EPL], accv[EPL];
-    load_row<T, EPL>(k1 + b * p.k1.b + (long)jb * p.k1.n + hk * p.k1.h, D, lane, k1v);
-    load_row<T, EPL>(v1 + b * p.v1.b + (long)jb * p.v1.n + hk * p.v1.h, D, lane, v1v);
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) { acck[e] = 0.f; accv[e] = 0.f; }
+// dK1 and dV1.  A cluster owns 32 K1/V1 rows of one KV head; its blocks take the tiles of 64 virtual rows that see them
+// (every query head of the group) in turn and add up their sums through distributed shared memory, in a fixed order.
+template <typename T, int DP>
+__global__ void __launch_bounds__(kThreads)
+bwd_col_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2, const T* __restrict__ v1,
+               const T* __restrict__ v2, const T* __restrict__ o, const float* __restrict__ lse, const T* __restrict__ d_o,
+               T* __restrict__ dk1, T* __restrict__ dv1) {
+    using S = Shape<DP>;
+    constexpr int PP = S::kColPPitch, V = S::kVec, NV = S::kDpt / V, NC = kColRows / 16;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int nrank = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    extern __shared__ __align__(16) float sm[];
+    float *As = sm, *Cs = As + S::kRowTile, *Ks = Cs + S::kRowTile, *Vs = Ks + kColRows * S::kPitch;
+    float *Ps = Vs + kColRows * S::kPitch, *Ds = Ps + kRows * PP, *st = Ds + kRows * PP;
+    int *ri = (int*)st, *rk = ri + kRows, *rh = rk + kRows;
+    float *delta = st + 3 * kRows, *L = delta + kRows;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int item = (int)(blockIdx.x / nrank), njt = (p.n1 + kColRows - 1) / kColRows;
+    const int j0 = (item % njt) * kColRows, hk = item / njt % p.Hkv, b = item / njt / p.Hkv;
+    const int nj = min(kColRows, p.n1 - j0);
     const T* k2h = k2 + b * p.k2.b + hk * p.k2.h;
     const T* v2h = v2 + b * p.v2.b + hk * p.v2.h;
-    const int i_lo = max(0, jb - p.halo1), i_hi = min(p.N - 1, jb - p.halo1 + p.w1 - 1);
-    for (int hq = 0; hq < p.G; ++hq) {
-        const int h = hk * p.G + hq;
-        for (int i = i_lo; i <= i_hi; ++i) {
-            float qv[EPL], dov[EPL], delta, L;
-            load_query<T, EPL>(p, q, o, d_o, lse, b, h, i, lane, qv, dov, delta, L);
-            const int k_hi = i + p.halo2, k_lo = max(0, k_hi - p.w2 + 1);
-            for (int k = k_lo; k <= k_hi; ++k) {
-                float a[EPL], c[EPL];
-                load_row<T, EPL>(k2h + (long)k * p.k2.n, D, lane, a, p.k2_bias);
-                load_row<T, EPL>(v2h + (long)k * p.v2.n, D, lane, c, p.v2_bias);
+    load_rows<T, DP>(Ks, k1 + b * p.k1.b + hk * p.k1.h, p.k1.n, j0, kColRows, nj, p.D);
+    load_rows<T, DP>(Vs, v1 + b * p.v1.b + hk * p.v1.h, p.v1.n, j0, kColRows, nj, p.D);
+    float ak[2][S::kDpt], av[2][S::kDpt];               // rows 2 ty, 2 ty + 1 of dK1, dV1
 #pragma unroll
-                for (int e = 0; e < EPL; ++e) { a[e] *= qv[e] * p.scale; c[e] *= dov[e]; }
-                const float s = warp_sum(dot<EPL>(a, k1v));
-                const float dP = warp_sum(dot<EPL>(c, v1v));
-                const float P = __expf(s - L);
-                const float dS = P * (dP - delta);
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-                for (int e = 0; e < EPL; ++e) { acck[e] = fmaf(dS, a[e], acck[e]); accv[e] = fmaf(P, c[e], accv[e]); }
+        for (int e = 0; e < S::kDpt; ++e) ak[a][e] = av[a][e] = 0.f;
+    const int i_lo = max(0, j0 - p.halo1), i_hi = min(p.N - 1, j0 + nj - 1 - p.halo1 + p.w1 - 1);
+    const int ni = max(0, i_hi - i_lo + 1);
+    const long total = (long)p.G * ni * p.w2;           // virtual rows, numbered (head, query, delta)
+    for (long v0 = (long)rank * kRows; v0 < total; v0 += (long)nrank * kRows) {
+        __syncthreads();
+        if (tid < kRows) {
+            const long v = v0 + tid;
+            const int dlt = (int)(v % p.w2), i = i_lo + (int)(v / p.w2 % ni), hq = (int)(v / p.w2 / ni), kb = i + p.halo2 - dlt;
+            ri[tid] = v < total && kb >= 0 ? i : -1;
+            rk[tid] = kb;
+            rh[tid] = hk * p.G + (v < total ? hq : 0);
+        }
+        __syncthreads();
+        // (as form_rows, with a head for every row)
+        bool bad = false;
+#pragma unroll 8
+        for (int idx = tid; idx < kRows * DP; idx += kThreads) {
+            const int r = idx / DP, d = idx % DP, i = ri[r], h = rh[r];
+            float a = 0.f, c = 0.f;
+            if (i >= 0 && d < p.D) {
+                a = to_f<T>(q[b * p.q.b + h * p.q.h + (int64_t)i * p.q.n + d]) * (to_f<T>(k2h[(int64_t)rk[r] * p.k2.n + d]) + p.k2_bias) * p.scale;
+                c = to_f<T>(d_o[b * p.d_o.b + h * p.d_o.h + (int64_t)i * p.d_o.n + d]) * (to_f<T>(v2h[(int64_t)rk[r] * p.v2.n + d]) + p.v2_bias);
+            }
+            bad |= not_finite(a) || not_finite(c);
+            As[r * S::kPitch + d] = a;
+            Cs[r * S::kPitch + d] = c;
+        }
+        row_stats<T>(delta, L, ri, o, p.o.n, d_o, p.d_o.n, lse, p.D, [&](int r, int what) -> int64_t {
+            const int h = rh[r];
+            return what == 0 ? b * p.o.b + h * p.o.h : what == 1 ? b * p.d_o.b + h * p.d_o.h : ((int64_t)b * p.H + h) * p.N;
+        });
+        const bool check = __syncthreads_or(bad);
+        float s[4][NC], dp[4][NC];
+        product<DP, NC>(As, Ks, ty, tx, s);
+        product<DP, NC>(Cs, Vs, ty, tx, dp);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            int lo, hi;
+            window(p, ri[4 * ty + a], j0, lo, hi);
+            const float la = L[4 * ty + a], de = delta[4 * ty + a];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const bool ok = tx + 16 * c >= lo && tx + 16 * c <= hi;
+                const float pv = ok ? __expf(s[a][c] - la) : 0.f;
+                Ps[(4 * ty + a) * PP + tx + 16 * c] = pv;
+                Ds[(4 * ty + a) * PP + tx + 16 * c] = ok ? pv * (dp[a][c] - de) : 0.f;
             }
         }
+        __syncthreads();
+        auto add = [&](auto check_c) {
+            constexpr bool CHECK = decltype(check_c)::value;
+#pragma unroll 4
+            for (int r = 0; r < kRows; ++r) {
+                float w[2], z[2];
+                lds_vec<2>(Ps + r * PP + 2 * ty, w);
+                lds_vec<2>(Ds + r * PP + 2 * ty, z);
+                int lo = 0, hi = kColRows;
+                if (CHECK) window(p, ri[r], j0, lo, hi);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    float x[V], y[V];
+                    lds_vec<V>(As + r * S::kPitch + tx * V + 16 * V * v, x);
+                    lds_vec<V>(Cs + r * S::kPitch + tx * V + 16 * V * v, y);
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) {
+                        if (CHECK && (2 * ty + a < lo || 2 * ty + a > hi)) continue;      // (as in accumulate)
+#pragma unroll
+                        for (int e = 0; e < V; ++e) {
+                            ak[a][V * v + e] = fmaf(z[a], x[e], ak[a][V * v + e]);
+                            av[a][V * v + e] = fmaf(w[a], y[e], av[a][V * v + e]);
+                        }
+                    }
+                }
+            }
+        };
+        if (check) add(std::true_type{});
+        else add(std::false_type{});
     }
-    if (dk1) store_row<T, EPL>(dk1 + b * p.dk1.b + (long)jb * p.dk1.n + hk * p.dk1.h, D, lane, acck);
-    if (dv1) store_row<T, EPL>(dv1 + b * p.dv1.b + (long)jb * p.dv1.n + hk * p.dv1.h, D, lane, accv);
-}
-
-// dK2 and dV2: warp per (b, hkv, K2 buffer row).
-template <typename T, int EPL>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-bwd_kv2_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, const T* __restrict__ k2,
-               const T* __restrict__ v1, const T* __restrict__ v2, const T* __restrict__ o,
-               const float* __restrict__ lse, const T* __restrict__ d_o, T* __restrict__ dk2, T* __restrict__ dv2) {
-    const long row = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= (long)p.B * p.Hkv * p.n2) return;
-    const int kb = (int)(row % p.n2);
-    const int hk = (int)((row / p.n2) % p.Hkv);
-    const int b = (int)(row / p.n2 / p.Hkv);
-    const int D = p.D;
-    float k2v[EPL], v2v[EPL], acck[EPL], accv[EPL];
-    load_row<T, EPL>(k2 + b * p.k2.b + (long)kb * p.k2.n + hk * p.k2.h, D, lane, k2v, p.k2_bias);
-    load_row<T, EPL>(v2 + b * p.v2.b + (long)kb * p.v2.n + hk * p.v2.h, D, lane, v2v, p.v2_bias);
+    __syncthreads();
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) { acck[e] = 0.f; accv[e] = 0.f; }
-    const T* k1h = k1 + b * p.k1.b + hk * p.k1.h;
-    const T* v1h = v1 + b * p.v1.b + hk * p.v1.h;
-    const int i_lo = max(0, kb - p.halo2), i_hi = min(p.N - 1, kb - p.halo2 + p.w2 - 1);
-    for (int hq = 0; hq < p.G; ++hq) {
-        const int h = hk * p.G + hq;
-        for (int i = i_lo; i <= i_hi; ++i) {
-            float qv[EPL], dov[EPL], delta, L;
-            load_query<T, EPL>(p, q, o, d_o, lse, b, h, i, lane, qv, dov, delta, L);
-            float a[EPL], c[EPL], g[EPL], u[EPL];
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int e = 0; e < EPL; ++e) { a[e] = qv[e] * k2v[e] * p.scale; c[e] = dov[e] * v2v[e]; g[e] = 0.f; u[e] = 0.f; }
-            const int j_hi = i + p.halo1, j_lo = max(0, j_hi - p.w1 + 1);
-            for (int j = j_lo; j <= j_hi; ++j) {
-                float k1v[EPL], v1v[EPL];
-                load_row<T, EPL>(k1h + (long)j * p.k1.n, D, lane, k1v);
-                load_row<T, EPL>(v1h + (long)j * p.v1.n, D, lane, v1v);
-                const float s = warp_sum(dot<EPL>(a, k1v));
-                const float dP = warp_sum(dot<EPL>(c, v1v));
-                const float P = __expf(s - L);
-                const float dS = P * (dP - delta);
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) { g[e] = fmaf(dS, k1v[e], g[e]); u[e] = fmaf(P, v1v[e], u[e]); }
-            }
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) {
-                acck[e] = fmaf(g[e], qv[e] * p.scale, acck[e]);
-                accv[e] = fmaf(u[e], dov[e], accv[e]);
-            }
+        for (int e = 0; e < S::kDpt; ++e) {
+            const int d = (e / V) * 16 * V + tx * V + e % V;
+            As[(2 * ty + a) * S::kPitch + d] = ak[a][e];
+            Cs[(2 * ty + a) * S::kPitch + d] = av[a][e];
+        }
+    cluster.sync();
+    const int rows = kColRows / nrank;                  // this block's share of the 32 rows
+    for (int idx = tid; idx < rows * DP; idx += kThreads) {
+        const int j = rank * rows + idx / DP, d = idx % DP;
+        float a = 0.f, c = 0.f;
+        for (int x = 0; x < nrank; ++x) {
+            a += cluster.map_shared_rank(As, x)[j * S::kPitch + d];
+            c += cluster.map_shared_rank(Cs, x)[j * S::kPitch + d];
+        }
+        if (j < nj && d < p.D) {
+            if (dk1) dk1[b * p.dk1.b + (int64_t)(j0 + j) * p.dk1.n + hk * p.dk1.h + d] = from_f<T>(a);
+            if (dv1) dv1[b * p.dv1.b + (int64_t)(j0 + j) * p.dv1.n + hk * p.dv1.h + d] = from_f<T>(c);
         }
     }
-    if (dk2) store_row<T, EPL>(dk2 + b * p.dk2.b + (long)kb * p.dk2.n + hk * p.dk2.h, D, lane, acck);
-    if (dv2) store_row<T, EPL>(dv2 + b * p.dv2.b + (long)kb * p.dv2.n + hk * p.dv2.h, D, lane, accv);
+    cluster.sync();                                     // the other blocks may still read this one's sums
 }
 
-template <typename T, int EPL>
+// Consecutive owners whose virtual rows fill a tile; a problem too small to give every multiprocessor a block is cut
+// finer.
+inline int owners_per_block(const KParams& p, long n_own, long heads, int sm_count) {
+    int n = kRows / p.w2 < 1 ? 1 : kRows / p.w2 > kMaxOwners ? kMaxOwners : kRows / p.w2;
+    while (n > 1 && (long)p.B * heads * ((n_own + n - 1) / n) < sm_count) n = (n + 1) / 2;
+    return n;
+}
+
+template <typename T, int DP>
 cudaError_t launch_fwd_t(const KParams& p, const void* q, const void* k1, const void* k2, const void* v1,
-                         const void* v2, void* o, float* lse, cudaStream_t st) {
-    const long rows = (long)p.B * p.H * p.N;
-    const unsigned blocks = (unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    fwd_kernel<T, EPL><<<blocks, kWarpsPerBlock * 32, 0, st>>>(p, (const T*)q, (const T*)k1, (const T*)k2,
-                                                               (const T*)v1, (const T*)v2, (T*)o, lse);
+                         const void* v2, void* o, float* lse, int sm_count, cudaStream_t st) {
+    const int owners = owners_per_block(p, p.N, p.H, sm_count);
+    const long blocks = (long)p.B * p.H * ((p.N + owners - 1) / owners);
+    if (!allow_dynamic_smem((const void*)fwd_kernel<T, DP>, Shape<DP>::kFwdBytes)) return cudaErrorInvalidValue;
+    fwd_kernel<T, DP><<<(unsigned)blocks, kThreads, Shape<DP>::kFwdBytes, st>>>(p, owners, (const T*)q, (const T*)k1, (const T*)k2,
+                                                                                (const T*)v1, (const T*)v2, (T*)o, lse);
     return cudaGetLastError();
 }
 
-template <typename T, int EPL>
+template <typename T, int DP>
 cudaError_t launch_bwd_t(const KParams& p, const void* q, const void* k1, const void* k2, const void* v1,
                          const void* v2, const void* o, const float* lse, const void* d_o, void* dq, void* dk1,
-                         void* dk2, void* dv1, void* dv2, cudaStream_t st) {
-    const int th = kWarpsPerBlock * 32;
-    auto nblk = [](long rows) { return (unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock); };
+                         void* dk2, void* dv1, void* dv2, int sm_count, cudaStream_t st) {
+    using S = Shape<DP>;
     if (dq) {
-        bwd_dq_kernel<T, EPL><<<nblk((long)p.B * p.H * p.N), th, 0, st>>>(
-            p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o, (T*)dq);
+        const int owners = owners_per_block(p, p.N, p.H, sm_count);
+        auto kern = bwd_row_kernel<T, DP, false>;
+        if (!allow_dynamic_smem((const void*)kern, S::kBwdBytes)) return cudaErrorInvalidValue;
+        kern<<<(unsigned)((long)p.B * p.H * ((p.N + owners - 1) / owners)), kThreads, S::kBwdBytes, st>>>(
+            p, owners, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o, (T*)dq,
+            (T*)nullptr, (T*)nullptr);
     }
     if (dk1 || dv1) {
-        bwd_kv1_kernel<T, EPL><<<nblk((long)p.B * p.Hkv * p.n1), th, 0, st>>>(
-            p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o,
-            (T*)dk1, (T*)dv1);
+        auto kern = bwd_col_kernel<T, DP>;
+        if (!allow_dynamic_smem((const void*)kern, S::kColBytes)) return cudaErrorInvalidValue;
+        const long items = (long)p.B * p.Hkv * ((p.n1 + kColRows - 1) / kColRows);
+        // blocks per cluster: enough of them for every multiprocessor, as long as each has tiles to work on
+        const long tiles = ((long)p.G * (p.w1 + kColRows < p.N ? p.w1 + kColRows : p.N) * p.w2 + kRows - 1) / kRows;
+        int nrank = 1;
+        while (nrank < 8 && items * nrank * 2 <= 2L * sm_count && nrank * 2 <= tiles) nrank *= 2;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(items * nrank));
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = S::kColBytes;
+        cfg.stream = st;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)nrank;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2,
+                                                 (const T*)o, lse, (const T*)d_o, (T*)dk1, (T*)dv1);
+        if (e != cudaSuccess) return e;
     }
     if (dk2 || dv2) {
-        bwd_kv2_kernel<T, EPL><<<nblk((long)p.B * p.Hkv * p.n2), th, 0, st>>>(
-            p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o,
-            (T*)dk2, (T*)dv2);
+        const int owners = owners_per_block(p, p.n2, p.Hkv, sm_count);
+        auto kern = bwd_row_kernel<T, DP, true>;
+        if (!allow_dynamic_smem((const void*)kern, S::kBwdBytes)) return cudaErrorInvalidValue;
+        kern<<<(unsigned)((long)p.B * p.Hkv * ((p.n2 + owners - 1) / owners)), kThreads, S::kBwdBytes, st>>>(
+            p, owners, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o,
+            (T*)nullptr, (T*)dk2, (T*)dv2);
     }
     return cudaGetLastError();
 }
 
-// Dispatch on dtype and head dim (elements per lane = ceil(D / 32)).
+// Dispatch on dtype and head dim (padded to 32, 64, 128 or 256).
 #define SA_GENERAL_DISPATCH(FN, ...)                                                         \
     do {                                                                                     \
         const int epl = (p.D + 31) / 32;                                                     \
         const int key = dtype * 16 + (epl <= 1 ? 1 : epl <= 2 ? 2 : epl <= 4 ? 4 : 8);       \
         switch (key) {                                                                       \
-            case 0 * 16 + 1: return FN<__nv_bfloat16, 1>(__VA_ARGS__);                       \
-            case 0 * 16 + 2: return FN<__nv_bfloat16, 2>(__VA_ARGS__);                       \
-            case 0 * 16 + 4: return FN<__nv_bfloat16, 4>(__VA_ARGS__);                       \
-            case 0 * 16 + 8: return FN<__nv_bfloat16, 8>(__VA_ARGS__);                       \
-            case 1 * 16 + 1: return FN<__half, 1>(__VA_ARGS__);                              \
-            case 1 * 16 + 2: return FN<__half, 2>(__VA_ARGS__);                              \
-            case 1 * 16 + 4: return FN<__half, 4>(__VA_ARGS__);                              \
-            case 1 * 16 + 8: return FN<__half, 8>(__VA_ARGS__);                              \
-            case 2 * 16 + 1: return FN<float, 1>(__VA_ARGS__);                               \
-            case 2 * 16 + 2: return FN<float, 2>(__VA_ARGS__);                               \
-            case 2 * 16 + 4: return FN<float, 4>(__VA_ARGS__);                               \
-            case 2 * 16 + 8: return FN<float, 8>(__VA_ARGS__);                               \
+            case 0 * 16 + 1: return FN<__nv_bfloat16, 32>(__VA_ARGS__);                      \
+            case 0 * 16 + 2: return FN<__nv_bfloat16, 64>(__VA_ARGS__);                      \
+            case 0 * 16 + 4: return FN<__nv_bfloat16, 128>(__VA_ARGS__);                     \
+            case 0 * 16 + 8: return FN<__nv_bfloat16, 256>(__VA_ARGS__);                     \
+            case 1 * 16 + 1: return FN<__half, 32>(__VA_ARGS__);                             \
+            case 1 * 16 + 2: return FN<__half, 64>(__VA_ARGS__);                             \
+            case 1 * 16 + 4: return FN<__half, 128>(__VA_ARGS__);                            \
+            case 1 * 16 + 8: return FN<__half, 256>(__VA_ARGS__);                            \
+            case 2 * 16 + 1: return FN<float, 32>(__VA_ARGS__);                              \
+            case 2 * 16 + 2: return FN<float, 64>(__VA_ARGS__);                              \
+            case 2 * 16 + 4: return FN<float, 128>(__VA_ARGS__);                             \
+            case 2 * 16 + 8: return FN<float, 256>(__VA_ARGS__);                             \
             default: return cudaErrorInvalidValue;                                           \
         }                                                                                    \
     } while (0)
 
 inline cudaError_t launch_fwd(int dtype, const KParams& p, const void* q, const void* k1, const void* k2,
-                              const void* v1, const void* v2, void* o, float* lse, cudaStream_t st) {
-    SA_GENERAL_DISPATCH(launch_fwd_t, p, q, k1, k2, v1, v2, o, lse, st);
+                              const void* v1, const void* v2, void* o, float* lse, int sm_count, cudaStream_t st) {
+    SA_GENERAL_DISPATCH(launch_fwd_t, p, q, k1, k2, v1, v2, o, lse, sm_count, st);
 }
 
 inline cudaError_t launch_bwd(int dtype, const KParams& p, const void* q, const void* k1, const void* k2,
                               const void* v1, const void* v2, const void* o, const float* lse, const void* d_o,
-                              void* dq, void* dk1, void* dk2, void* dv1, void* dv2, cudaStream_t st) {
-    SA_GENERAL_DISPATCH(launch_bwd_t, p, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, st);
+                              void* dq, void* dk1, void* dk2, void* dv1, void* dv2, int sm_count, cudaStream_t st) {
+    SA_GENERAL_DISPATCH(launch_bwd_t, p, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, sm_count, st);
 }
 
 }  // namespace general

@@ -487,3 +487,56 @@ def test_projection_module_matches_oracle_and_trains():
     for prm in (mod.in_proj.weight, mod.out_proj.weight):
         assert prm.grad is not None and bool(torch.isfinite(prm.grad.float()).all()) and float(prm.grad.float().abs().sum()) > 0
     assert x.grad is not None and x.grad.shape == x.shape
+
+
+# B, N, H, Hkv, D, w1, w2, k2_bias, v2_bias, halo1, halo2: head dims at the edges of the padded ones, K2 windows around
+# the 64 virtual rows of a tile, one and many queries to a tile, K1 windows around a tile's columns
+GENERAL_CASES = [
+    (1, 1, 1, 1, 8, 1, 1, 0.0, 0.0, 0, 0),
+    (1, 37, 2, 1, 33, 17, 3, 0.1, -0.1, 0, 0),
+    (2, 70, 3, 3, 32, 64, 64, 0.0, 0.0, 0, 0),
+    (1, 150, 2, 2, 40, 65, 65, 0.0, 0.0, 0, 0),
+    (1, 140, 4, 2, 96, 16, 24, 0.0, 0.2, 15, 23),
+    (1, 90, 1, 1, 130, 33, 16, 0.0, 0.0, 0, 0),
+    (1, 200, 2, 1, 200, 80, 130, 0.0, 0.0, 0, 0),
+    (1, 75, 1, 1, 256, 100, 7, 0.1, 0.0, 0, 0),
+    (3, 600, 4, 4, 64, 128, 2, 0.0, 0.0, 0, 0),
+]
+
+
+@pytest.mark.parametrize("case", GENERAL_CASES)
+def test_general_kernels_vs_cpu_oracle_fp32(case):
+    """The oracle in fp64; fp32 sums of at most w1 * w2 terms of order 1 in another order: 1e-5 relative."""
+    B, N, H, Hkv, D, w1, w2, kb, vb, h1, h2 = case
+    ts = so.make_inputs(B, N, H, Hkv, D, seed=13, seed_do=14, halo1=h1, halo2=h2)
+    scale = 1.0 / math.sqrt(D)
+    cfg = dict(w1=w1, w2=w2, scale=scale, k2_bias=kb, v2_bias=vb)
+    o, lse, grads = _run(dict(zip(("q", "k1", "k2", "v1", "v2", "do"), ts)), cfg, "general", dtype=torch.float32, halo1=h1, halo2=h2)
+    ref = so.forward_backward(*ts, w1, w2, scale, kb, vb, h1, h2, dtype=torch.float64)
+    assert so.rel_l2(o.cpu().double(), ref[0]) <= 1e-5
+    assert float((lse.cpu() - ref[1]).abs().max()) <= 1e-5
+    for nm, g, r in zip(("dq", "dk1", "dk2", "dv1", "dv2"), grads, ref[2:]):
+        if float(r.abs().max()) < 1e-12:      # one (j, k) pair to a query: no gradient of the scores
+            assert float(g.abs().max()) <= 1e-4, nm
+        else:
+            assert so.rel_l2(g.cpu().double(), r) <= 1e-5, nm
+
+
+def test_general_kernels_keep_values_that_are_not_finite_to_their_windows():
+    """An infinity in one row of an input reaches the results of the queries that see it, and of the rows that those
+    see, and no others, although tiles hold rows of several windows: everything else equals the run on finite inputs."""
+    B, N, H, D, w1, w2 = 1, 160, 1, 32, 40, 8
+    ts = dict(zip(("q", "k1", "k2", "v1", "v2", "do"), so.make_inputs(B, N, H, H, D, seed=21, seed_do=22)))
+    cfg = dict(w1=w1, w2=w2, scale=1.0 / math.sqrt(D), k2_bias=0.0, v2_bias=0.0)
+    clean = _run(ts, cfg, "general", dtype=torch.float32)
+    x = 70
+    for name, last in (("k1", x + w1 - 1), ("v1", x + w1 - 1), ("k2", x + w2 - 1), ("v2", x + w2 - 1), ("q", x), ("do", x)):
+        bad = dict(ts)
+        bad[name] = ts[name].clone()
+        bad[name][0, x, 0, 3] = float("inf")
+        o, _, grads = _run(bad, cfg, "general", dtype=torch.float32)
+        for got, want, behind in [(o, clean[0], 0), (grads[0], clean[2][0], 0), (grads[1], clean[2][1], w1 - 1), (grads[2], clean[2][2], w2 - 1),
+                                  (grads[3], clean[2][3], w1 - 1), (grads[4], clean[2][4], w2 - 1)]:
+            far = torch.ones(N, dtype=torch.bool)
+            far[max(0, x - behind):last + 1] = False
+            assert torch.equal(got[:, far], want[:, far]), name
