@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "sa_common.cuh"
 
 namespace sa {
@@ -475,6 +477,15 @@ __device__ __forceinline__ void mma_ts_lo(uint32_t leader, uint32_t d_tmem, uint
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader), "n"(kDescHi), "n"(OFFA), "n"(OFFB)
         : "memory");
 }
+// Calls f with the integral constants 0 .. N - 1: a loop whose index can be a template argument.
+template <int N, typename F, int I = 0>
+__device__ __forceinline__ void static_for(F&& f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        static_for<N, F, I + 1>(static_cast<F&&>(f));
+    }
+}
+
 // Low word of a K-major (lbo 16) or MN-major (lbo: bytes between 64-element slabs) descriptor.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
     return ((smem_addr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16);

@@ -31,7 +31,7 @@
 // groups turn a buffer into P and dS (16-bit, in place) while the tensor cores work on the other buffer
 // (bwd_row_kernel: one group per buffer; bwd_row2_kernel: both groups split every tile's columns); P and dS
 // then feed the two accumulating MMAs from tensor memory.  Column kernel: one 128-column S^T / dP^T pair,
-// both softmax groups split its columns and hand P^T / dS^T to the MMA warp in 16-column chunks.
+// both softmax groups split its columns and hand P^T, later dS^T, to the MMA warp in two parts.
 #pragma once
 
 #include <type_traits>
@@ -252,7 +252,7 @@ struct ColSmem {
     static constexpr int kStream = 2 * kTile;
     static constexpr int kMeta = kStream + kColStages * 2 * kTile;
     static constexpr int kBars = kMeta + kColStages * 256 * 4;
-    static constexpr int kNumBars = 2 * kColStages + 10;
+    static constexpr int kNumBars = 4 * kColStages + 12;
     static constexpr int kMisc = kBars + kNumBars * 8;
     static constexpr int kTotal = kMisc + 16;
     static constexpr int kAlloc = (kTotal + 1024 > 120 * 1024) ? kTotal + 1024 : 120 * 1024;
@@ -260,14 +260,23 @@ struct ColSmem {
 
 // One streamed tile covers 128 virtual rows, so S^T and dP^T are single 128x128 tiles: the MMAs run
 // with N = 128 (a 128x64 tile costs almost as much: the 128-row stationary operand is re-read from
-// shared memory either way) and in long bursts.  S^T / dP^T are not double buffered (tensor memory
-// is full: 128 + 128 + 2 x 128 accumulator columns); instead both softmax groups work on the same
-// tile, group g on columns [64g, 64g + 64), and write P / dS back inside their own column range.
+// shared memory either way).  S^T / dP^T are not double buffered (tensor memory is full: 128 + 128 +
+// 2 x 128 accumulator columns); instead the two halves of a tile's work are staggered.  The MMA order is
+//     ... dK1(t-1)  dP(t)  dV1(t)  S(t+1)  dK1(t)  dP(t+1) ...
+// and the softmax groups (group g: columns [64g, 64g + 64)) alternate between P(t) from S(t), kept in
+// registers in fp32, and dS(t) from dP(t): the exponentials of a tile run under dK1(t-1) and dP(t), its dS
+// under dV1(t) and S(t+1), so neither side waits for a whole chain of the other.
+// Bound by the softmax groups (exponentials: 1024 cycles per tile at 16 per clock, measured 2000 with their loads,
+// stores and hand-overs, plus 880 for dS) and the issue of the SS MMAs (100 cycles each while the producers store the
+// next tiles, 64 without), 3700 cycles per tile where the whole chain per tile took 4300.  Measured, us, before ->
+// after: B1 N16384 H32/2 D128 w 512/32 11706 -> 9690; B1 N8192 H16 D128 w 1024/64 10558 -> 9010; B4 N2048 H16 D64
+// w 64/64 1449 -> 1217; B2 N512 H4 D64 w 32/32 89 -> 78; at short windows with 16 deltas, where every tile is half masked
+// and the producers set the pace, it costs: B4 N8192 H16 D128 w 128/16 2555 -> 2843 (3067 with 96 registers for them).
 // Registers per thread of the column kernel's softmax groups, producers and remaining warps (multiples of 8).
 #ifndef SA_COL_SM
-#define SA_COL_SM 96
+#define SA_COL_SM 112
 #define SA_COL_PR 112
-#define SA_COL_REST 64
+#define SA_COL_REST 32
 #endif
 static_assert(128 * (2 * SA_COL_SM + 2 * SA_COL_PR + SA_COL_REST) <= 640 * 96 && SA_COL_SM >= 96 && SA_COL_PR >= 96,
               "register pool of the column kernel's block");
@@ -285,14 +294,18 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
     const uint32_t smem_base = smem_u32(smem);
     const KParams& p = P.k;
     uint64_t* bars = (uint64_t*)(smem + L::kBars);
-    uint64_t* st_full = bars;                         // [kColStages] A and C of a tile formed (256 arrivals)
-    uint64_t* st_empty = bars + kColStages;           // [kColStages] tile consumed (commit)
-    uint64_t* sdp_ready = bars + 2 * kColStages;      // S^T, dP^T computed (commit)
-    uint64_t* pds_ready = sdp_ready + 6;              // [4] P^T, dS^T of the k-th 16-column chunk of both groups stored (256 arrivals)
-    uint64_t* stat_full = sdp_ready + 2;              // K1, V1 landed (TMA)
-    uint64_t* stat_empty = sdp_ready + 3;             // K1, V1 no longer read (commit)
-    uint64_t* acc_ready = sdp_ready + 4;              // dV1, dK1 final (commit)
-    uint64_t* acc_free = sdp_ready + 5;               // dV1, dK1 read out (256 arrivals)
+    uint64_t* a_full = bars;                          // [kColStages] A of a tile formed, its LSE2 and Delta stored (4 warps)
+    uint64_t* a_empty = a_full + kColStages;          // [kColStages] A consumed (commit)
+    uint64_t* c_full = a_empty + kColStages;          // [kColStages] C of a tile formed (4 warps)
+    uint64_t* c_empty = c_full + kColStages;          // [kColStages] C consumed (commit)
+    uint64_t* s_ready = c_empty + kColStages;         // S^T computed (commit)
+    uint64_t* dp_ready = s_ready + 1;                 // dP^T computed (commit)
+    uint64_t* p_ready = s_ready + 2;                  // [2] P^T of the k-th 32 columns of both groups stored (8 warps)
+    uint64_t* ds_ready = s_ready + 4;                 // [2] dS^T likewise
+    uint64_t* stat_full = s_ready + 6;                // [2] K1, V1 landed (TMA)
+    uint64_t* stat_empty = s_ready + 8;               // [2] K1, V1 no longer read (commit)
+    uint64_t* acc_ready = s_ready + 10;               // dV1, dK1 final (commit)
+    uint64_t* acc_free = s_ready + 11;                // dV1, dK1 read out (8 warps)
     uint32_t* tmem_slot = (uint32_t*)(smem + L::kMisc);
     volatile int* abort_flag = (volatile int*)(smem + L::kMisc + 4);
     const WaitCtx wctx{smem_u32((const void*)abort_flag), P.status, P.wait_limit_ns};
@@ -302,13 +315,19 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
     SA_TR_DECL();
     if (tid == 0) {
         for (int s = 0; s < kColStages; ++s) {
-            mbar_init(&st_full[s], 8);         // one arrival per producer warp
-            mbar_init(&st_empty[s], 1);
+            mbar_init(&a_full[s], 4);          // one arrival per producer warp of the group
+            mbar_init(&a_empty[s], 1);
+            mbar_init(&c_full[s], 4);
+            mbar_init(&c_empty[s], 1);
         }
-        mbar_init(sdp_ready, 1);
-        for (int k = 0; k < 4; ++k) mbar_init(&pds_ready[k], 8);      // one arrival per softmax warp
-        mbar_init(stat_full, 1);
-        mbar_init(stat_empty, 1);
+        mbar_init(s_ready, 1);
+        mbar_init(dp_ready, 1);
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&p_ready[k], 8);         // one arrival per softmax warp
+            mbar_init(&ds_ready[k], 8);
+            mbar_init(&stat_full[k], 1);
+            mbar_init(&stat_empty[k], 1);
+        }
         mbar_init(acc_ready, 1);
         mbar_init(acc_free, 8);
         *abort_flag = 0;
@@ -344,81 +363,101 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
             const int nt = ci.ntq * p.G;
             for (int t = 0; t < nt; ++t) {
                 const uint32_t g = g_base + t;
-                const int stage = (int)(g % kColStages);
-                const float* m_lse = (const float*)(smem + L::kMeta) + stage * 256;
+                const float* m_lse = (const float*)(smem + L::kMeta) + (g % kColStages) * 256;
                 const float* m_delta = m_lse + 128;
-                const long rho0 = (long)(ci.tt_lo + (t % ci.ntq)) * kColTileRows;
-                const int iq0 = (int)(rho0 >> P.dw_log2);
-                mbar_wait(sdp_ready, g & 1, wctx, 20);
-                if ((warp & 3) == 0) SA_TR(1 + grp, 52);
-                tc_fence_after();
-                SA_PROF_T0(t_csm);
-                if (P.dw_log2 >= 4) {
-                    // 16 columns (virtual rows) at a time, each chunk within one query; the next chunk's
-                    // tensor-memory loads are in flight while the current one is processed.  A step whose
-                    // columns all lie inside the window of every row of the warp needs no masks.
-                    const int i_first = (int)((rho0 + 64 * grp) >> P.dw_log2), i_last = (int)((rho0 + 64 * grp + 63) >> P.dw_log2);
-                    const bool step_full = __all_sync(0xffffffffu, jb <= i_first + p.halo1 && jb >= i_last + p.halo1 - p.w1 + 1);
-                    auto run_step = [&](auto masked_tag) {
-                        constexpr bool MASKED = decltype(masked_tag)::value;
-                        uint32_t s[2][16], dp[2][16];
-                        tmem_ld16(tm_s + lane_addr + 64 * grp, s[0]);
-                        tmem_ld16(tm_dp + lane_addr + 64 * grp, dp[0]);
+                // query x of the tile (x = column >> dw_log2: a tile starts with a whole query) sees this row if
+                // x_lo <= x <= x_hi; a warp whose rows are seen by every query of its columns needs no masks
+                const int iq0 = (int)(((long)(ci.tt_lo + (t % ci.ntq)) * kColTileRows) >> P.dw_log2);
+                const int x_lo = jb - p.halo1 - iq0, x_hi = x_lo + p.w1 - 1;
+                const bool full = __all_sync(0xffffffffu, x_lo <= (64 * grp) >> P.dw_log2 && x_hi >= (64 * grp + 63) >> P.dw_log2);
+                // MODE 0: no masks; 1: 16 columns belong to one query; 2: every column may be another query
+                auto step = [&](auto mode_tag) {
+                    constexpr int MODE = decltype(mode_tag)::value;
+                    uint32_t pr[2][32];                  // S, then P (fp32) of the group's 64 columns of this lane
+                    mbar_wait(s_ready, g & 1, wctx, 20);
+                    if ((warp & 3) == 0) SA_TR(1 + grp, 52);
+                    tc_fence_after();
+                    tmem_ld32(tm_s + lane_addr + 64 * grp, pr[0]);
+                    tmem_ld32(tm_s + lane_addr + 64 * grp + 32, pr[1]);
+                    tmem_wait_ld();
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int c0 = 64 * grp + 16 * k;
-                            tmem_wait_ld();
-                            if (k + 1 < 4) {
-                                tmem_ld16(tm_s + lane_addr + c0 + 16, s[(k + 1) & 1]);
-                                tmem_ld16(tm_dp + lane_addr + c0 + 16, dp[(k + 1) & 1]);
+                    for (int k = 0; k < 2; ++k) {
+                        uint32_t pp[16];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int c0 = 64 * grp + 32 * k + 16 * h;
+                            const int x = c0 >> P.dw_log2;
+                            const float nl = -m_lse[x];
+                            const bool valid = MODE == 0 || (x >= x_lo && x <= x_hi);
+#pragma unroll
+                            for (int e = 0; e < 16; e += 2) {
+                                uint32_t& r0 = pr[k][16 * h + e];
+                                uint32_t& r1 = pr[k][16 * h + e + 1];
+                                float2 y;
+                                if constexpr (MODE < 2) {
+                                    y = __ffma2_rn(make_float2(__uint_as_float(r0), __uint_as_float(r1)), make_float2(c2, c2), make_float2(nl, nl));
+                                    y = make_float2(ex2(y.x), ex2(y.y));
+                                    if (MODE == 1) y = make_float2(valid ? y.x : 0.f, valid ? y.y : 0.f);
+                                } else {
+                                    const int xa = (c0 + e) >> P.dw_log2, xb = (c0 + e + 1) >> P.dw_log2;
+                                    y.x = ex2(fmaf(__uint_as_float(r0), c2, -m_lse[xa]));
+                                    y.y = ex2(fmaf(__uint_as_float(r1), c2, -m_lse[xb]));
+                                    y = make_float2(xa >= x_lo && xa <= x_hi ? y.x : 0.f, xb >= x_lo && xb <= x_hi ? y.y : 0.f);
+                                }
+                                r0 = __float_as_uint(y.x);
+                                r1 = __float_as_uint(y.y);
+                                pp[8 * h + (e >> 1)] = E::pack(y.x, y.y);
                             }
-                            const int i = (int)((rho0 + c0) >> P.dw_log2);
-                            const bool valid = !MASKED || ((jb <= i + p.halo1) && (jb >= i + p.halo1 - p.w1 + 1));
-                            uint32_t pp[8], ds[8];
-                            softmax_bwd_chunk<MASKED, 16, F16>(s[k & 1], dp[k & 1], 0, valid ? 0 : 1, valid ? 15 : 0, c2, m_lse[i - iq0],
-                                                          m_delta[i - iq0], pp, ds);
-                            // packed P^T / dS^T of columns [64g + 16k, +16) go to tensor-memory columns 64g + 8k ...
-                            tmem_st8(tm_s + lane_addr + 64 * grp + 8 * k, pp);
-                            tmem_st8(tm_dp + lane_addr + 64 * grp + 8 * k, ds);
-                            // the accumulating MMAs of this chunk start while the next one is processed
-                            tmem_wait_st();
-                            tc_fence_before();
-                            warp_arrive(&pds_ready[k]);
                         }
-                    };
-                    if (step_full) run_step(std::false_type{});
-                    else run_step(std::true_type{});
-                } else {
-#pragma unroll 1
-                    for (int cc = 0; cc < 64; cc += 16) {
-                        const int c0 = 64 * grp + cc;
-                        uint32_t s[16], dp[16], pp[8], ds[8];
-                        tmem_ld16(tm_s + lane_addr + c0, s);
-                        tmem_ld16(tm_dp + lane_addr + c0, dp);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < 16; e += 2) {
-                            float pv[2], dv[2];
-#pragma unroll
-                            for (int x = 0; x < 2; ++x) {
-                                const int i = (int)((rho0 + c0 + e + x) >> P.dw_log2);
-                                const bool valid = (jb <= i + p.halo1) && (jb >= i + p.halo1 - p.w1 + 1);
-                                const float pe = ex2(fmaf(__uint_as_float(s[e + x]), c2, -m_lse[i - iq0]));
-                                pv[x] = valid ? pe : 0.f;
-                                dv[x] = valid ? pe * (__uint_as_float(dp[e + x]) - m_delta[i - iq0]) : 0.f;
-                            }
-                            pp[e >> 1] = E::pack(pv[0], pv[1]);
-                            ds[e >> 1] = E::pack(dv[0], dv[1]);
-                        }
-                        tmem_st8(tm_s + lane_addr + 64 * grp + (cc >> 1), pp);
-                        tmem_st8(tm_dp + lane_addr + 64 * grp + (cc >> 1), ds);
+                        // packed P^T of columns [64g + 32k, +32) go to tensor-memory columns 64g + 16k ...: the MMAs that
+                        // read them start while the next ones are processed
+                        tmem_st16(tm_s + lane_addr + 64 * grp + 16 * k, pp);
                         tmem_wait_st();
                         tc_fence_before();
-                        warp_arrive(&pds_ready[cc >> 4]);
+                        warp_arrive(&p_ready[k]);
                     }
-                }
-                SA_PROF_ADD(28, t_csm);
-                if ((warp & 3) == 0) SA_TR(1 + grp, 53);
+                    mbar_wait(dp_ready, g & 1, wctx, 28);
+                    if ((warp & 3) == 0) SA_TR(1 + grp, 54);
+                    tc_fence_after();
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        uint32_t dp[2][16], ds[16];
+                        tmem_ld16(tm_dp + lane_addr + 64 * grp + 32 * k, dp[0]);
+                        tmem_ld16(tm_dp + lane_addr + 64 * grp + 32 * k + 16, dp[1]);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int c0 = 64 * grp + 32 * k + 16 * h;
+                            const int x = c0 >> P.dw_log2;
+                            const float nd = -m_delta[x];
+                            const bool valid = MODE == 0 || (x >= x_lo && x <= x_hi);
+#pragma unroll
+                            for (int e = 0; e < 16; e += 2) {
+                                const float2 y = make_float2(__uint_as_float(pr[k][16 * h + e]), __uint_as_float(pr[k][16 * h + e + 1]));
+                                const float2 z = make_float2(__uint_as_float(dp[h][e]), __uint_as_float(dp[h][e + 1]));
+                                float2 d;
+                                // (a masked column is selected away, never multiplied: its dP may be anything)
+                                if constexpr (MODE < 2) {
+                                    d = __fmul2_rn(y, __fadd2_rn(z, make_float2(nd, nd)));
+                                    if (MODE == 1) d = make_float2(valid ? d.x : 0.f, valid ? d.y : 0.f);
+                                } else {
+                                    const int xa = (c0 + e) >> P.dw_log2, xb = (c0 + e + 1) >> P.dw_log2;
+                                    d.x = xa >= x_lo && xa <= x_hi ? y.x * (z.x - m_delta[xa]) : 0.f;
+                                    d.y = xb >= x_lo && xb <= x_hi ? y.y * (z.y - m_delta[xb]) : 0.f;
+                                }
+                                ds[8 * h + (e >> 1)] = E::pack(d.x, d.y);
+                            }
+                        }
+                        tmem_st16(tm_dp + lane_addr + 64 * grp + 16 * k, ds);
+                        tmem_wait_st();
+                        tc_fence_before();
+                        warp_arrive(&ds_ready[k]);
+                    }
+                    if ((warp & 3) == 0) SA_TR(1 + grp, 53);
+                };
+                if (P.dw_log2 < 4) step(std::integral_constant<int, 2>{});
+                else if (full) step(std::integral_constant<int, 0>{});
+                else step(std::integral_constant<int, 1>{});
             }
             g_base += nt;
             // epilogue: group 0 writes dV1, group 1 writes dK1 (times scale)
@@ -502,7 +541,7 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
                 const int h = ci.hk * p.G + t / ci.ntq;
                 const long rho0 = (long)(ci.tt_lo + (t % ci.ntq)) * kColTileRows;
                 uint8_t* tile = smem + L::kStream + (stage * 2 + grp) * L::kTile;
-                mbar_wait(&st_empty[stage], ((g / kColStages) & 1) ^ 1, wctx, 22);
+                mbar_wait(grp == 0 ? &a_empty[stage] : &c_empty[stage], ((g / kColStages) & 1) ^ 1, wctx, 22);
                 if ((warp & 3) == 0) SA_TR(3 + grp, 50);
                 SA_PROF_T0(t_cform);
                 const float bias = BIAS ? (grp == 0 ? p.k2_bias : p.v2_bias) : 0.f;
@@ -521,7 +560,7 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
                     m_lse[128 + row] = meta_delta;
                 }
                 fence_proxy_async_smem();
-                warp_arrive(&st_full[stage]);
+                warp_arrive(grp == 0 ? &a_full[stage] : &c_full[stage]);
                 if ((warp & 3) == 0) SA_TR(3 + grp, 51);
                 SA_PROF_ADD(37 + grp, t_cform);
                 // the next tile's rows start travelling now (past the item's end: this tile's once more, never used, so
@@ -549,64 +588,75 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
             uint32_t g_base = 0, n_items = 0;
             const uint32_t idesc_sd = make_idesc(128, kColTileRows, false, false, F16);
             const uint32_t idesc_acc = make_idesc(128, HD, false, true, F16);
-            const uint64_t d_k1 = desc_kmajor(smem_base + L::kK1, 0), d_v1 = desc_kmajor(smem_base + L::kV1, 0);
+            // (low words of the operands' descriptors; the high words are constants)
+            const uint32_t d_k1 = desc_lo(smem_base + L::kK1, 16), d_v1 = desc_lo(smem_base + L::kV1, 16);
+            const uint32_t d_a0 = desc_lo(smem_base + L::kStream, 16), d_am0 = desc_lo(smem_base + L::kStream, L::kSlab);
+            constexpr uint32_t kC = L::kTile >> 4, kStage = 2 * L::kTile >> 4;       // from A to C, from stage to stage
+            // one of the two products of a tile with the block's rows: X Y^T, X the rows, Y the streamed tile
+            auto product = [&](uint32_t dst, uint32_t x, uint32_t y) {
+                static_for<HD / 16>([&](auto kk_c) {
+                    constexpr int kk = decltype(kk_c)::value, off = ((kk >> 2) * L::kSlab + (kk & 3) * 32) >> 4;
+                    mma_ss_lo<off, off>(leader, dst, x, y, idesc_sd, kk > 0);
+                });
+            };
+            // 32 columns of each softmax group (k-steps 2k, 2k + 1 and 4 + 2k, 5 + 2k): acc += W^T-tile Y-tile
+            auto accumulate = [&](auto k_c, uint32_t acc, uint32_t w, uint32_t y, bool add) {
+                constexpr int k = decltype(k_c)::value;
+                static_for<4>([&](auto x_c) {
+                    constexpr int x = decltype(x_c)::value, gq = x >> 1, c = 2 * k + (x & 1);
+                    mma_ts_lo<gq * 64 + c * 8, (4 * gq + c) * (2048 >> 4)>(leader, acc, w, y, idesc_acc, add || k > 0 || x > 0);
+                });
+            };
             for (long it = blockIdx.x; it < P.num_col_items; it += gridDim.x) {
                 const ColItem ci = col_item(P, it);
                 const int nt = ci.ntq * p.G;
                 if (nt == 0) continue;
-                mbar_wait(stat_full, n_items & 1, wctx, 23);
-                if (n_items > 0) mbar_wait(acc_free, (n_items - 1) & 1, wctx, 24);
-                tc_fence_after();
+                mbar_wait(&stat_full[0], n_items & 1, wctx, 23);
                 for (int t = 0; t < nt; ++t) {
-                    const uint32_t g = g_base + t;
-                    const int stage = (int)(g % kColStages);
-                    const uint32_t a_t = smem_base + L::kStream + stage * 2 * L::kTile, c_t = a_t + L::kTile;
-                    const uint64_t d_a = desc_kmajor(a_t, 0), d_c = desc_kmajor(c_t, 0);
-                    const uint64_t d_am = desc_mnmajor(a_t, L::kSlab), d_cm = desc_mnmajor(c_t, L::kSlab);
+                    const uint32_t g = g_base + t, stage = g % kColStages, par = (g / kColStages) & 1;
+                    if (t == 0) {
+                        mbar_wait(&a_full[stage], par, wctx, 25);
+                        tc_fence_after();
+                        product(tm_s, d_k1, d_a0 + stage * kStage);                  // S^T = K1 A^T
+                        tc_commit(leader, s_ready);
+                        if (nt == 1) tc_commit(leader, &stat_empty[0]);
+                        mbar_wait(&stat_full[1], n_items & 1, wctx, 23);
+                    }
                     SA_TR(0, 1);
-                    mbar_wait(&st_full[stage], (g / kColStages) & 1, wctx, 25);
+                    mbar_wait(&c_full[stage], par, wctx, 29);
                     SA_TR(0, 2);
                     tc_fence_after();
-                    // S^T = K1 A^T,  dP^T = V1 C^T
-                    SA_PROF_T0(t_ci1);
-#pragma unroll
-                    for (int kk = 0; kk < HD / 16; ++kk) {
-                        const uint32_t off = ((kk >> 2) * L::kSlab + (kk & 3) * 32) >> 4;
-                        mma_ss(leader, tm_s, d_k1 + off, d_a + off, idesc_sd, kk > 0);
-                    }
-#pragma unroll
-                    for (int kk = 0; kk < HD / 16; ++kk) {
-                        const uint32_t off = ((kk >> 2) * L::kSlab + (kk & 3) * 32) >> 4;
-                        mma_ss(leader, tm_dp, d_v1 + off, d_c + off, idesc_sd, kk > 0);
-                    }
-                    tc_commit(leader, sdp_ready);
+                    product(tm_dp, d_v1, d_a0 + stage * kStage + kC);                // dP^T = V1 C^T
+                    tc_commit(leader, dp_ready);
+                    if (t == nt - 1) tc_commit(leader, &stat_empty[1]);              // the block's last read of V1
+                    if (t == 0 && n_items > 0) mbar_wait(acc_free, (n_items - 1) & 1, wctx, 24);
                     SA_TR(0, 3);
-                    SA_PROF_ADD(29, t_ci1);
-                    SA_PROF_T0(t_ci2);
-                    // dV1 += P^T-tile C-tile,  dK1 += dS^T-tile A-tile   (K = 128 virtual rows: 8 steps of 16).
-                    // Chunk k of both softmax groups (k-steps k and 4 + k) is issued as soon as it is stored.
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        mbar_wait(&pds_ready[k], g & 1, wctx, 26);
-                        SA_TR(0, 10 + k);
+                    static_for<2>([&](auto k_c) {                                    // dV1 += P^T-tile C-tile
+                        mbar_wait(&p_ready[decltype(k_c)::value], g & 1, wctx, 26);
+                        SA_TR(0, 10);
                         tc_fence_after();
-#pragma unroll
-                        for (int gq = 0; gq < 2; ++gq) {
-                            const int kk = 4 * gq + k;
-                            mma_ts(leader, tm_dv1, tm_s + gq * 64 + k * 8, d_cm + kk * (2048 >> 4), idesc_acc, t > 0 || k > 0 || gq > 0);
-                        }
-#pragma unroll
-                        for (int gq = 0; gq < 2; ++gq) {
-                            const int kk = 4 * gq + k;
-                            mma_ts(leader, tm_dk1, tm_dp + gq * 64 + k * 8, d_am + kk * (2048 >> 4), idesc_acc, t > 0 || k > 0 || gq > 0);
-                        }
+                        accumulate(k_c, tm_dv1, tm_s, d_am0 + stage * kStage + kC, t > 0);
+                    });
+                    tc_commit(leader, &c_empty[stage]);
+                    if (t + 1 < nt) {
+                        const uint32_t stage1 = (g + 1) % kColStages;
+                        mbar_wait(&a_full[stage1], ((g + 1) / kColStages) & 1, wctx, 25);
+                        SA_TR(0, 5);
+                        tc_fence_after();
+                        product(tm_s, d_k1, d_a0 + stage1 * kStage);
+                        tc_commit(leader, s_ready);
+                        if (t + 2 == nt) tc_commit(leader, &stat_empty[0]);          // ... of K1
                     }
-                    tc_commit(leader, &st_empty[stage]);
+                    static_for<2>([&](auto k_c) {                                    // dK1 += dS^T-tile A-tile
+                        mbar_wait(&ds_ready[decltype(k_c)::value], g & 1, wctx, 36);
+                        SA_TR(0, 11);
+                        tc_fence_after();
+                        accumulate(k_c, tm_dk1, tm_dp, d_am0 + stage * kStage, t > 0);
+                    });
+                    tc_commit(leader, &a_empty[stage]);
                     SA_TR(0, 4);
-                    SA_PROF_ADD(36, t_ci2);
                 }
                 tc_commit(leader, acc_ready);
-                tc_commit(leader, stat_empty);
                 g_base += nt;
                 ++n_items;
             }
@@ -622,12 +672,13 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
             for (long it = blockIdx.x; it < P.num_col_items; it += gridDim.x) {
                 const ColItem ci = col_item(P, it);
                 if (ci.ntq == 0) continue;
-                mbar_wait(stat_empty, (n & 1) ^ 1, wctx, 27);
-                mbar_arrive_expect_tx(stat_full, 2 * L::kTile);
+#pragma unroll 1
+                for (int kv = 0; kv < 2; ++kv) {
+                    mbar_wait(&stat_empty[kv], (n & 1) ^ 1, wctx, 27);
+                    mbar_arrive_expect_tx(&stat_full[kv], L::kTile);
 #pragma unroll
-                for (int sl = 0; sl < L::kSlabs; ++sl) {
-                    tma_load_4d(smem + L::kK1 + sl * L::kSlab, &map_k1, stat_full, sl * 64, ci.j0, ci.hk, ci.b);
-                    tma_load_4d(smem + L::kV1 + sl * L::kSlab, &map_v1, stat_full, sl * 64, ci.j0, ci.hk, ci.b);
+                    for (int sl = 0; sl < L::kSlabs; ++sl)
+                        tma_load_4d(smem + (kv ? L::kV1 : L::kK1) + sl * L::kSlab, kv ? &map_v1 : &map_k1, &stat_full[kv], sl * 64, ci.j0, ci.hk, ci.b);
                 }
                 ++n;
             }
@@ -1905,6 +1956,7 @@ int launch_bwd_t(const KParams& k, const void* q, const void* k1, const void* k2
 // The two element types are compiled in translation units of their own (sa_tc_bwd_bf16.cu, sa_tc_bwd_f16.cu: the
 // kernels of one type take minutes to compile, and the units build side by side); everywhere else the
 // instantiations are only declared.
+#ifndef SA_TC_BWD_UNIT
 #ifndef SA_TC_BWD_INSTANTIATE
 extern template int launch_bwd_t<false>(const KParams&, const void*, const void*, const void*, const void*, const void*, const void*,
                                         const float*, const void*, void*, void*, void*, void*, void*, uint8_t*, DeviceStatus*,
@@ -1923,6 +1975,7 @@ inline int launch_bwd(const KParams& k, const void* q, const void* k1, const voi
                : launch_bwd_t<false>(k, q, k1, k2, v1, v2, o, lse, d_o, dq, dk1, dk2, dv1, dv2, workspace, status, st, nlaunch,
                                      make_map, sm_count, wait_limit_ns);
 }
+#endif
 
 }  // namespace tc
 }  // namespace sa

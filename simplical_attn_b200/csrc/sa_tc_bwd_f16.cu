@@ -5,7 +5,7 @@
 
 #include "../../include/simplicial_attn_b200.h"
 #include "sa_common.cuh"
-#define SA_TC_BWD_INSTANTIATE
+#define SA_TC_BWD_UNIT
 #include "sa_tc_bwd.cuh"
 
 namespace sa {

@@ -160,14 +160,6 @@ struct RingPos {
     }
 };
 
-template <int N, typename F, int I = 0>
-__device__ __forceinline__ void static_for(F&& f) {
-    if constexpr (I < N) {
-        f(std::integral_constant<int, I>{});
-        static_for<N, F, I + 1>(static_cast<F&&>(f));
-    }
-}
-
 // BIAS = false: both biases are zero, every bias add folds away.  F16: the tensors are IEEE half instead of bf16
 // (same kernels; only the element encoding and the MMA's operand format differ).  The head dim may be smaller than
 // HD (a multiple of 8): TMA fills the missing columns with zeros and they are not written out.
