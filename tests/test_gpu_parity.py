@@ -540,3 +540,21 @@ def test_general_kernels_keep_values_that_are_not_finite_to_their_windows():
             far = torch.ones(N, dtype=torch.bool)
             far[max(0, x - behind):last + 1] = False
             assert torch.equal(got[:, far], want[:, far]), name
+
+
+@pytest.mark.parametrize("N", [3, 5, 9, 17])
+def test_backward_of_many_short_sequences(N):
+    """More K1/V1 row tiles than multiprocessors, one to a few tiles of 128 virtual rows to each: the hand-overs of
+    the stationary rows and accumulators from one row tile to the next, with next to no tiles between them; and,
+    with four sequences, a column kernel that fills less than half of the GPU beside the row kernel."""
+    H, D, w1, w2 = 4, 64, 12, 16
+    for B in (4, 100):
+        ts = so.make_inputs(B, N, H, H, D, seed=31, seed_do=32)
+        scale = 1.0 / math.sqrt(D)
+        cfg = dict(w1=w1, w2=w2, scale=scale, k2_bias=0.0, v2_bias=0.0)
+        o, _, grads = _run(dict(zip(("q", "k1", "k2", "v1", "v2", "do"), ts)), cfg, "tcgen05")
+        ref = so.forward_backward(*ts, w1, w2, scale)
+        # (relative: next to no averaging, so |O| reaches 10 and one bf16 rounding of it 10 * 2^-9)
+        assert so.rel_l2(o.float().cpu(), ref[0]) <= TOL_G_BF16
+        for nm, g, r in zip(("dq", "dk1", "dk2", "dv1", "dv2"), grads, ref[2:]):
+            assert _grad_err(g, r) <= TOL_G_BF16, nm
