@@ -371,13 +371,32 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
                 const int iq0 = (int)(((long)(ci.tt_lo + (t % ci.ntq)) * kColTileRows) >> P.dw_log2);
                 const int x_lo = jb - p.halo1 - iq0, x_hi = x_lo + p.w1 - 1;
                 const bool full = __all_sync(0xffffffffu, x_lo <= (64 * grp) >> P.dw_log2 && x_hi >= (64 * grp + 63) >> P.dw_log2);
-                // MODE 0: no masks; 1: 16 columns belong to one query; 2: every column may be another query
+                mbar_wait(s_ready, g & 1, wctx, 20);
+                if ((warp & 3) == 0) SA_TR(1 + grp, 52);
+                tc_fence_after();
+                // Padding rows (delta >= w2, or no such K2 row) have zero operand rows, so their P = e^-LSE and dS = -P Delta
+                // add nothing: as long as both are finite in 16 bits (inf * 0 is NaN).  Where a query's are not, the P of its
+                // padding is masked (and with it dS).
+                bool pad = false;
+                if (p.w2 < 1 << P.dw_log2 || iq0 + p.halo2 < (1 << P.dw_log2) - 1) {
+                    auto large = [&](int c) {
+                        const int x = c >> P.dw_log2;
+                        return !(ex2(-m_lse[x]) * fmaxf(1.f, fabsf(m_delta[x])) <= (F16 ? 60000.f : 3e38f));
+                    };
+                    pad = __any_sync(0xffffffffu, large(64 * grp + lane) || large(64 * grp + 32 + lane));
+                }
+                // MODE 0: no masks; 1: 16 columns belong to one query; 2: every column may be another query, or padding
                 auto step = [&](auto mode_tag) {
                     constexpr int MODE = decltype(mode_tag)::value;
+                    uint32_t keep[2] = {0u, 0u};         // MODE 2: a bit per column that is no padding
+                    if constexpr (MODE == 2) {
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int c = 64 * grp + 32 * k + lane, x = c >> P.dw_log2, delta = c - (x << P.dw_log2);
+                            keep[k] = __ballot_sync(0xffffffffu, delta < p.w2 && iq0 + x + p.halo2 >= delta);
+                        }
+                    }
                     uint32_t pr[2][32];                  // S, then P (fp32) of the group's 64 columns of this lane
-                    mbar_wait(s_ready, g & 1, wctx, 20);
-                    if ((warp & 3) == 0) SA_TR(1 + grp, 52);
-                    tc_fence_after();
                     tmem_ld32(tm_s + lane_addr + 64 * grp, pr[0]);
                     tmem_ld32(tm_s + lane_addr + 64 * grp + 32, pr[1]);
                     tmem_wait_ld();
@@ -403,7 +422,8 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
                                     const int xa = (c0 + e) >> P.dw_log2, xb = (c0 + e + 1) >> P.dw_log2;
                                     y.x = ex2(fmaf(__uint_as_float(r0), c2, -m_lse[xa]));
                                     y.y = ex2(fmaf(__uint_as_float(r1), c2, -m_lse[xb]));
-                                    y = make_float2(xa >= x_lo && xa <= x_hi ? y.x : 0.f, xb >= x_lo && xb <= x_hi ? y.y : 0.f);
+                                    y.x = xa >= x_lo && xa <= x_hi && (keep[k] & (1u << (16 * h + e))) ? y.x : 0.f;
+                                    y.y = xb >= x_lo && xb <= x_hi && (keep[k] & (2u << (16 * h + e))) ? y.y : 0.f;
                                 }
                                 r0 = __float_as_uint(y.x);
                                 r1 = __float_as_uint(y.y);
@@ -456,7 +476,7 @@ bwd_col_kernel(const __grid_constant__ BwdTcParams P, const __grid_constant__ CU
                     }
                     if ((warp & 3) == 0) SA_TR(1 + grp, 53);
                 };
-                if (P.dw_log2 < 4) step(std::integral_constant<int, 2>{});
+                if (pad || P.dw_log2 < 4) step(std::integral_constant<int, 2>{});
                 else if (full) step(std::integral_constant<int, 0>{});
                 else step(std::integral_constant<int, 1>{});
             }

@@ -558,3 +558,23 @@ def test_backward_of_many_short_sequences(N):
         assert so.rel_l2(o.float().cpu(), ref[0]) <= TOL_G_BF16
         for nm, g, r in zip(("dq", "dk1", "dk2", "dv1", "dv2"), grads, ref[2:]):
             assert _grad_err(g, r) <= TOL_G_BF16, nm
+
+
+@pytest.mark.parametrize("dtype,score", [(torch.float16, 15.0), (torch.bfloat16, 95.0)])
+@pytest.mark.parametrize("D,w2", [(64, 24), (128, 32), (64, 5), (128, 60)])
+def test_padding_rows_beside_a_query_of_low_scores(dtype, score, D, w2):
+    """Query 0 has one (j, k) pair, whose score is -`score`: e^-LSE does not fit 16 bits.  The virtual rows that only fill a
+    tile up (delta >= w2, K2 rows before the first) must not bring it into dK1 and dV1.
+
+    Rounding the D products Q * K2 of a score of that size to 16 bits changes it by up to eps * score, eps * score / sqrt(D)
+    where the roundings are independent, and P by as much (relative): that is added to the bf16 tolerance."""
+    N, w1, scale = 150, 40, 1.0 / math.sqrt(D)
+    ts = dict(zip(("q", "k1", "k2", "v1", "v2", "do"), so.make_inputs(1, N, 1, 1, D, seed=41, seed_do=42)))
+    z = (score / (D * scale)) ** (1 / 3)
+    ts["q"][0, 0], ts["k1"][0, 0], ts["k2"][0, 0] = z, -z, z
+    cfg = dict(w1=w1, w2=w2, scale=scale, k2_bias=0.0, v2_bias=0.0)
+    o, lse, grads = _run(ts, cfg, "tcgen05", dtype=dtype)
+    assert float(lse.flatten()[0]) < -score + 0.5
+    tol = TOL_G_BF16 + score / math.sqrt(D) * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
+    for nm, g, r in zip(("dq", "dk1", "dk2", "dv1", "dv2"), grads, _run(ts, cfg, "general", dtype=dtype)[2]):
+        assert bool(torch.isfinite(g).all()) and so.rel_l2(g.float().cpu(), r.float().cpu()) <= tol, nm
