@@ -421,9 +421,11 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
         const int wq = warp & 3;
         const uint32_t rb = smem_base + r * 8;
         const float v2_bias = BIAS ? p.v2_bias : 0.f;
-        // A tile of row tile r: row rho = (query rho / DW, delta rho % DW), a thread takes one 16-byte chunk of every
-        // RPP-th row.  Rows with delta >= w2 are zeros.
-        auto form = [&] {
+        // A tile of row tile r of the unit at query i0: row rho = (query rho / DW, delta rho % DW), a thread takes one
+        // 16-byte chunk of every RPP-th row.  Padding (delta >= w2, K2 rows before the first) repeats the query's last row:
+        // its scores and T are as finite as that row's, so that the merge's zero weight drops them.  (Zero rows would meet
+        // an infinity in K1 as NaN.)
+        auto form = [&](int i0) {
             constexpr int CH = HD / 8, RPP = 128 / CH;
             const int c = t % CH, row0 = t / CH;
             const uint32_t tile = smem_base + L::kA + r * L::kTileBytes + (c >> 3) * L::kSlabBytes;
@@ -431,12 +433,11 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
 #pragma unroll 4
             for (int k = 0; k < 128 / RPP; ++k) {
                 const int rho = row0 + k * RPP;
-                const int q2 = r * qpt + (rho >> P.dw_log2), dlt = rho & (DW - 1), wr = q2 + DW - 1 - dlt;
+                const int q2 = r * qpt + (rho >> P.dw_log2), dlt = min(rho & (DW - 1), min(p.w2 - 1, max(i0 + q2 + p.halo2, 0)));
+                const int wr = q2 + DW - 1 - dlt;
                 const uint4 x = lds128(qsl + q2 * 128 + (((c ^ q2) & 7) << 4));
                 const uint4 y = lds128(ksl + wr * 128 + (((c ^ wr) & 7) << 4));
-                uint4 v = BIAS ? mul_chunk<F16>(x, y, p.k2_bias) : mul_chunk_nobias<F16>(x, y);
-                if (dlt >= p.w2) v = make_uint4(0, 0, 0, 0);
-                sts128(tile + rho * 128 + (((c ^ rho) & 7) << 4), v);
+                sts128(tile + rho * 128 + (((c ^ rho) & 7) << 4), BIAS ? mul_chunk<F16>(x, y, p.k2_bias) : mul_chunk_nobias<F16>(x, y));
             }
             fence_proxy_async_smem();
             SA_FWD_ARRIVE(kAReady, rb);
@@ -486,7 +487,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
             SA_FWD_ARRIVE(kStFree, rb);           // m, l of this unit are no longer needed
 #pragma unroll
             for (int sft = sft0; sft >= 1; sft >>= 1) lq += __shfl_xor_sync(0xffffffffu, lq, sft);
-            const float wrow = e_own / lq;        // (rows that are not valid: 0, or never stored if the whole query is not)
+            const float wrow = m_own > -INFINITY ? e_own / lq : 0.f;
             {
                 const int i = i0 + (t >> P.dw_log2);
                 if ((t & (DW - 1)) == 0 && i < p.N) lse[((long)b * p.H + h) * p.N + i] = (mq + log2f(lq)) * kLn2;
@@ -498,9 +499,8 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
             for (int k = 0; k < 4; ++k) {
                 const int rl = (lane >> 2) + 8 * k, rr = 32 * wq + rl;
                 wk[k] = __shfl_sync(0xffffffffu, wrow, rl);
-                const bool ok = wk[k] > 0.f;
-                if (!ok) wk[k] = 0.f;
-                const int wr = r * qpt + (rr >> P.dw_log2) + DW - 1 - (rr & (DW - 1));
+                const int q2 = rr >> P.dw_log2, dlt = rr & (DW - 1), wr = r * qpt + q2 + DW - 1 - dlt;
+                const bool ok = i0 + q2 < p.N && dlt < p.w2 && i0 + q2 + p.halo2 >= dlt;
                 va[k] = (ok ? v2_st + wr * 128 + ((wr & 7) << 4) : smem_base + L::kZero) + (lane & 3) * 4;
                 sl[k] = ok ? win_slab : 0u;
             }
@@ -600,7 +600,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
             uint32_t nu = 0;
             if (w.valid(P)) {
                 mbar_wait<kQkFull>(smem_base, 0, wctx, 16);
-                form();
+                form(w.qb * qrows);
             }
             while (w.valid(P)) {
                 UnitWalk wn = w;
@@ -610,7 +610,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                     mbar_wait<kQkFull>(smem_base, (nu + 1) & 1, wctx, 16);
                     mbar_wait<kAFree>(rb, nu & 1, wctx, 11);
                     if (wq == 0) SA_TR(2 + r, 50);
-                    form();
+                    form(wn.qb * qrows);
                     if (wq == 0) SA_TR(2 + r, 52);
                 }
                 // ---- merge of this unit
@@ -639,8 +639,8 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
         if (r >= P.row_tiles) w.u = P.num_units;
         for (; w.valid(P); w.next(P), ++nu) {
             const UnitGeom ug = w.geom(P);
-            // valid buffer rows of this query: [jlo, jhi].  Rows that are not valid for another reason (delta >= w2, a
-            // K2 row before the buffer, a query past the end) run along with finite values: the merge drops them.
+            // valid buffer rows of this query: [jlo, jhi].  Padding rows (delta >= w2, a K2 row before the buffer, a query past
+            // the end) run along, and the merge drops them.
             const int jhi = ug.i0 + r * qpt + (row >> P.dw_log2) + p.halo1 - ug.col_start;
             const int jlo = max(-ug.col_start, jhi - p.w1 + 1);
             float m = -INFINITY, l = 0.f;

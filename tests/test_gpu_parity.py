@@ -578,3 +578,24 @@ def test_padding_rows_beside_a_query_of_low_scores(dtype, score, D, w2):
     tol = TOL_G_BF16 + score / math.sqrt(D) * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
     for nm, g, r in zip(("dq", "dk1", "dk2", "dv1", "dv2"), grads, _run(ts, cfg, "general", dtype=dtype)[2]):
         assert bool(torch.isfinite(g).all()) and so.rel_l2(g.float().cpu(), r.float().cpu()) <= tol, nm
+
+
+@pytest.mark.parametrize("D,w2", [(64, 24), (128, 32), (64, 5), (128, 60), (64, 1), (128, 100)])
+def test_forward_with_values_that_are_not_finite(D, w2):
+    """A K1 row of -inf in a column where Q * K2 is positive (a mask: its P is 0) leaves the output finite and equal to
+    that of the general kernels; a NaN or an infinity in Q, K2 or V2, or a NaN in K1, reaches the queries that see it
+    and no others."""
+    N, w1, x = 200, 40, 70
+    ts = dict(zip(("q", "k1", "k2", "v1", "v2"), so.make_inputs(1, N, 1, 1, D, seed=43, seed_do=44)))
+    for nm in ("q", "k2"):
+        ts[nm][..., 3] = ts[nm][..., 3].abs() + 0.125
+    for name, value in (("k1", -math.inf), ("q", math.nan), ("q", math.inf), ("k2", math.nan), ("v2", math.nan), ("v2", math.inf), ("k1", math.nan)):
+        bad = {nm: t.clone() for nm, t in ts.items()}
+        bad[name][0, x, 0, 3] = value
+        t = [bad[nm].to(DEV).to(torch.bfloat16) for nm in ("q", "k1", "k2", "v1", "v2")]
+        (o, lse), (want, want_lse) = (sab.two_simplicial_attn_fwd_kernel(*t, w1, w2, 1.0 / math.sqrt(D), algo=a) for a in ("tcgen05", "general"))
+        assert torch.equal(torch.isfinite(o).all(-1), torch.isfinite(want).all(-1)), (name, value)
+        fin = torch.isfinite(o) & torch.isfinite(want)
+        assert float((o.float() - want.float())[fin].abs().max()) <= 3e-2, (name, value)      # two bf16-rounded results
+        if value == -math.inf:
+            assert bool(fin.all()) and float((lse - want_lse).abs().max()) <= 2e-2
