@@ -6,10 +6,15 @@
 // word that is cleared on the device before and copied back after every call) that was 76 microseconds per
 // forward call at B1 H2 N256 D64 w 64/16.
 //
+// Only plain calls are made here: tensors that are torch.Tensor or Parameter themselves, and for the autograd node no
+// tracing, functorch transform or forward-mode tangent, which the Python autograd function records or refuses.  For
+// other calls the entry points return None and the Python layer takes over.
+//
 // Device-side timeouts: the kernels record them straight into a pinned host word per device and direction
 // (sa_forward_status / sa_backward_status), which every later call looks at before it launches.  Nothing is
 // cleared, copied or waited for per call.
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <Python.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -63,6 +68,8 @@ volatile int* slot(int device, Direction d) {
     }
     return base + (device * 2 + d) * kSlotInts;
 }
+
+void* status_word(int device, Direction d) { return const_cast<int*>(slot(device, d)); }
 
 PyObject* g_on_error = nullptr;       // Python callable (function name, status, detail or None) that raises
 
@@ -133,21 +140,12 @@ sa_params make_params(const Tensor& q, const Tensor& k1, const Tensor& k2, const
 
 constexpr size_t kStatusBytes = 256;      // the part of a workspace that a separate status word makes unnecessary
 
-// The caller's workspace if it gave one (its head is then the status word), else one from torch's allocator.
+// A workspace from torch's allocator, if the call needs more than the status word.
 struct Workspace {
     Tensor t;
     void* ptr = nullptr;
     size_t bytes = 0;
-    void* status = nullptr;
-    Workspace(const Tensor& given, size_t need, const Tensor& like, volatile int* status_slot) {
-        if (given.defined()) {
-            t = given;
-            ptr = t.data_ptr();
-            bytes = (size_t)t.numel();
-            status = ptr;
-            return;
-        }
-        status = const_cast<int*>(status_slot);
+    Workspace(size_t need, const Tensor& like) {
         if (need > kStatusBytes) {
             t = at::empty({(int64_t)need}, like.options().dtype(at::kByte));
             ptr = t.data_ptr();
@@ -157,7 +155,7 @@ struct Workspace {
 };
 
 std::pair<Tensor, Tensor> forward_call(const Tensor& q_, const Tensor& k1_, const Tensor& k2_, const Tensor& v1_, const Tensor& v2_,
-                                       const Config& c, const Tensor& given_ws) {
+                                       const Config& c) {
     const Tensor q = unit_inner(q_), k1 = unit_inner(k1_), k2 = unit_inner(k2_), v1 = unit_inner(v1_), v2 = unit_inner(v2_);
     check_inputs(q, k1, k2, v1, v2, c);
     const c10::cuda::CUDAGuard guard(q.device());
@@ -166,16 +164,17 @@ std::pair<Tensor, Tensor> forward_call(const Tensor& q_, const Tensor& k1_, cons
     Tensor o = at::empty_like(q);
     Tensor lse = at::empty({q.size(0), q.size(2), q.size(1)}, q.options().dtype(at::kFloat));
     const sa_params p = make_params(q, k1, k2, v1, v2, o, c);
-    const Workspace ws(given_ws, given_ws.defined() ? 0 : sa_forward_workspace_size(&p), q, slot(device, kForward));
+    const Workspace ws(sa_forward_workspace_size(&p), q);
     const int rc = sa_forward_status(&p, q.data_ptr(), k1.data_ptr(), k2.data_ptr(), v1.data_ptr(), v2.data_ptr(), o.data_ptr(),
-                                     (float*)lse.data_ptr(), ws.ptr, ws.bytes, ws.status, at::cuda::getCurrentCUDAStream(device).stream());
+                                     (float*)lse.data_ptr(), ws.ptr, ws.bytes, status_word(device, kForward),
+                                     at::cuda::getCurrentCUDAStream(device).stream());
     if (rc != SA_OK) raise_status("sa_forward", rc);
     return {std::move(o), std::move(lse)};
 }
 
 std::array<Tensor, 5> backward_call(const Tensor& q_, const Tensor& k1_, const Tensor& k2_, const Tensor& v1_, const Tensor& v2_,
                                     const Tensor& o_, const Tensor& lse, const Tensor& d_o_, const Config& c,
-                                    const std::array<bool, 5>& need, const Tensor& given_ws) {
+                                    const std::array<bool, 5>& need) {
     const Tensor q = unit_inner(q_), k1 = unit_inner(k1_), k2 = unit_inner(k2_), v1 = unit_inner(v1_), v2 = unit_inner(v2_),
                  o = unit_inner(o_), d_o = unit_inner(d_o_);
     check_inputs(q, k1, k2, v1, v2, c);
@@ -192,10 +191,10 @@ std::array<Tensor, 5> backward_call(const Tensor& q_, const Tensor& k1_, const T
     sa_params p = make_params(q, k1, k2, v1, v2, o, c);
     p.d_o = strides_of(d_o);
     p.dq = strides_of(g[0]); p.dk1 = strides_of(g[1]); p.dk2 = strides_of(g[2]); p.dv1 = strides_of(g[3]); p.dv2 = strides_of(g[4]);
-    const Workspace ws(given_ws, given_ws.defined() ? 0 : sa_backward_workspace_size(&p), q, slot(device, kBackward));
+    const Workspace ws(sa_backward_workspace_size(&p), q);
     const int rc = sa_backward_status(&p, q.data_ptr(), k1.data_ptr(), k2.data_ptr(), v1.data_ptr(), v2.data_ptr(), o.data_ptr(),
                                       (const float*)lse.data_ptr(), d_o.data_ptr(), gp[0], gp[1], gp[2], gp[3], gp[4], ws.ptr, ws.bytes,
-                                      ws.status, at::cuda::getCurrentCUDAStream(device).stream());
+                                      status_word(device, kBackward), at::cuda::getCurrentCUDAStream(device).stream());
     if (rc != SA_OK) raise_status("sa_backward", rc);
     return g;
 }
@@ -217,7 +216,7 @@ struct AttentionBackward : public torch::autograd::Node {
         const Tensor q_ = q.unpack(), k1_ = k1.unpack(), k2_ = k2.unpack(), v1_ = v1.unpack(), v2_ = v2.unpack(), o_ = o.unpack(self),
                      lse_ = lse.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
-        std::array<Tensor, 5> g = backward_call(q_, k1_, k2_, v1_, v2_, o_, lse_, grads[0], cfg, need, Tensor());
+        std::array<Tensor, 5> g = backward_call(q_, k1_, k2_, v1_, v2_, o_, lse_, grads[0], cfg, need);
         for (int i = 0; i < 5; ++i) out[i] = std::move(g[i]);
         return out;
     }
@@ -243,7 +242,7 @@ Tensor attention(const Tensor& q, const Tensor& k1, const Tensor& k2, const Tens
     std::pair<Tensor, Tensor> r;
     {
         at::AutoDispatchBelowADInplaceOrView below;
-        r = forward_call(q, k1, k2, v1, v2, c, Tensor());
+        r = forward_call(q, k1, k2, v1, v2, c);
     }
     if (node) {
         torch::autograd::set_history(r.first, node);
@@ -258,7 +257,6 @@ const Tensor& tensor_arg(PyObject* o, const char* name) {
     TORCH_CHECK_TYPE(THPVariable_Check(o), name, " must be a tensor");
     return THPVariable_Unpack(o);
 }
-Tensor optional_tensor(PyObject* o) { return o == Py_None ? Tensor() : tensor_arg(o, "workspace"); }
 int64_t int_arg(PyObject* o) {
     PyObject* l = PyNumber_Long(o);
     const int64_t v = l ? PyLong_AsLongLong(l) : -1;
@@ -284,11 +282,31 @@ Config config_args(PyObject* const* a) {
     c.algo = (int)int_arg(a[7]);
     return c;
 }
+// Whether every one of the five inputs is a torch.Tensor or Parameter itself: what a subclass does with the tensors that
+// are allocated for it is up to its __torch_function__.
+bool exact(PyObject* const* a) {
+    for (int i = 0; i < 5; ++i)
+        if (!THPVariable_CheckTypeExact(Py_TYPE(a[i]))) return false;
+    return true;
+}
+// ... and the call is neither traced nor under a functorch transform, and no input carries a forward-mode tangent.
+bool plain(PyObject* const* a) {
+    if (!exact(a) || at::tracer::impl::is_dispatch_enabled() ||
+        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+        return false;
+    for (int i = 0; i < 5; ++i) {
+        const Tensor& t = THPVariable_Unpack(a[i]);
+        if (t.unsafeGetTensorImpl()->autograd_meta() != nullptr && t._fw_grad(0).defined()) return false;
+    }
+    return true;
+}
+
 void expect(Py_ssize_t have, Py_ssize_t want) { TORCH_CHECK_TYPE(have == want, "expected ", want, " arguments, got ", have); }
 
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     expect(n, 13);
+    if (!plain(a)) Py_RETURN_NONE;
     const Config c = config_args(a + 5);
     const Tensor &q = tensor_arg(a[0], "q"), &k1 = tensor_arg(a[1], "k1"), &k2 = tensor_arg(a[2], "k2"), &v1 = tensor_arg(a[3], "v1"),
                  &v2 = tensor_arg(a[4], "v2");
@@ -303,16 +321,16 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    expect(n, 14);
+    expect(n, 13);
+    if (!exact(a)) Py_RETURN_NONE;
     const Config c = config_args(a + 5);
     const Tensor &q = tensor_arg(a[0], "q"), &k1 = tensor_arg(a[1], "k1"), &k2 = tensor_arg(a[2], "k2"), &v1 = tensor_arg(a[3], "v1"),
                  &v2 = tensor_arg(a[4], "v2");
-    const Tensor ws = optional_tensor(a[13]);
     std::pair<Tensor, Tensor> r;
     {
         pybind11::gil_scoped_release no_gil;
         at::AutoDispatchBelowADInplaceOrView below;
-        r = forward_call(q, k1, k2, v1, v2, c, ws);
+        r = forward_call(q, k1, k2, v1, v2, c);
     }
     PyObject* t = PyTuple_New(2);
     PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(r.first)));
@@ -321,23 +339,23 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// q, k1, k2, v1, v2, o, lse, d_o, <8 configuration values>, need (bit i: gradient i), workspace
+// q, k1, k2, v1, v2, o, lse, d_o, <8 configuration values>, need (bit i: gradient i)
 PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    expect(n, 18);
+    expect(n, 17);
+    if (!exact(a)) Py_RETURN_NONE;
     static const char* const names[8] = {"q", "k1", "k2", "v1", "v2", "o", "lse", "d_o"};
     const Tensor* t[8];
     for (int i = 0; i < 8; ++i) t[i] = &tensor_arg(a[i], names[i]);
     const Config c = config_args(a + 8);
     const int64_t bits = int_arg(a[16]);
-    const Tensor ws = optional_tensor(a[17]);
     std::array<bool, 5> need;
     for (int i = 0; i < 5; ++i) need[i] = (bits >> i) & 1;
     std::array<Tensor, 5> g;
     {
         pybind11::gil_scoped_release no_gil;
         at::AutoDispatchBelowADInplaceOrView below;
-        g = backward_call(*t[0], *t[1], *t[2], *t[3], *t[4], *t[5], *t[6], *t[7], c, need, ws);
+        g = backward_call(*t[0], *t[1], *t[2], *t[3], *t[4], *t[5], *t[6], *t[7], c, need);
     }
     PyObject* r = PyTuple_New(5);
     for (int i = 0; i < 5; ++i) {
@@ -345,6 +363,13 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         else PyTuple_SET_ITEM(r, i, Py_NewRef(Py_None));
     }
     return r;
+    END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect(n, 5);
+    return PyBool_FromLong(plain(a));
     END_HANDLE_TH_ERRORS
 }
 
@@ -374,9 +399,10 @@ PyObject* py_on_error(PyObject*, PyObject* fn) {
 }
 
 PyMethodDef kMethods[] = {
-    {"attention", (PyCFunction)(void*)py_attention, METH_FASTCALL, "O with its autograd history"},
-    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "(O, LSE)"},
-    {"backward", (PyCFunction)(void*)py_backward, METH_FASTCALL, "(dq, dk1, dk2, dv1, dv2)"},
+    {"attention", (PyCFunction)(void*)py_attention, METH_FASTCALL, "O with its autograd history; None if the call is not plain"},
+    {"plain", (PyCFunction)(void*)py_plain, METH_FASTCALL, "whether `attention` makes the call for these five inputs"},
+    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "(O, LSE); None for tensor subclasses"},
+    {"backward", (PyCFunction)(void*)py_backward, METH_FASTCALL, "(dq, dk1, dk2, dv1, dv2); None for tensor subclasses"},
     {"poll", py_poll, METH_O, "raises if an earlier call on the device left a status"},
     {"devices", py_devices, METH_NOARGS, "indices of the devices that have been called on"},
     {"on_error", py_on_error, METH_O, "sets the callable that raises for a status"},

@@ -4,8 +4,9 @@ Same names, argument meaning and return values as the reference's
 `simplicial/triton_impl.py` (`TwoSimplicialAttentionFunction`, :15-158; `TwoSimplicialAttention`,
 :161-186); the Triton launches are replaced by calls through the C ABI of
 libsimplicial_attn_b200.so, made by a native binding (`binding/sa_torch.cpp`: argument checks, output
-allocation, autograd node) so that a small problem is not bound by Python.  torch supplies device memory
-and the current stream, nothing else.
+allocation, autograd node) so that a small problem is not bound by Python.  Calls that are not plain
+(tensor subclasses, `torch.jit.trace`, functorch, forward-mode tangents) are made from here, through ctypes
+and a Python autograd function.  torch supplies device memory and the current stream, nothing else.
 
 Additions that keep the reference call signature valid:
   * K/V may have fewer heads than Q (`H % Hkv == 0`); query head h reads KV head h // (H // Hkv).
@@ -41,6 +42,27 @@ def _ptr(t: Optional[torch.Tensor]):
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
+def _check_inputs(q, k1, k2, v1, v2, halo1, halo2):
+    if not q.is_cuda:
+        raise RuntimeError("simplical_attn_b200 runs on CUDA tensors only; there is no CPU path")
+    if q.dim() != 4:
+        raise ValueError("q must be [batch, seq_len, num_heads, head_dim]")
+    B, N, H, D = q.shape
+    if q.dtype not in _DTYPES:
+        raise TypeError(f"unsupported dtype {q.dtype}")
+    for name, t, halo in (("k1", k1, halo1), ("v1", v1, halo1), ("k2", k2, halo2), ("v2", v2, halo2)):
+        if t.dtype != q.dtype or t.device != q.device:
+            raise TypeError(f"{name} must match q's dtype and device")
+        if t.dim() != 4 or t.shape[0] != B or t.shape[1] != N + halo or t.shape[3] != D:
+            raise ValueError(f"{name} must be [batch, seq_len + halo, kv_heads, head_dim], got {tuple(t.shape)}")
+        if t.shape[2] != k1.shape[2] or H % t.shape[2] != 0:
+            raise ValueError("K/V tensors must share a head count that divides the query head count")
+
+
+def _unit_inner(t: torch.Tensor) -> torch.Tensor:
+    return t if t.stride(-1) == 1 else t.contiguous()
+
+
 def _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo):
     B, N, H, D = q.shape
     p = _abi.Params()
@@ -59,15 +81,15 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
     return ws
 
 
-_default_workspace = _workspace       # where `_workspace` is replaced its buffers are used; otherwise the binding allocates
+_default_workspace = _workspace       # where `_workspace` is replaced its buffers are used, and the binding is not
 
 
 class _StatusWatch:
     """Surfaces device-side timeouts without a synchronisation per call.
 
-    A call without a workspace of its caller's has its kernels report into a pinned host word, which the
-    binding looks at before every launch.  A caller's workspace carries the status word itself: after the
-    launch it is copied, stream-ordered, into a pinned host slot and an event is recorded.  `poll()` looks
+    The binding's calls have their kernels report into a pinned host word, which it looks at before every
+    launch.  In the calls made from here the workspace carries the status word: after the launch it is
+    copied, stream-ordered, into a pinned host slot and an event is recorded.  `poll()` looks
     at the slots whose event has already completed (a non-blocking query) and raises if one of them holds
     an error.  `flush()` synchronises and checks everything that is still pending."""
 
@@ -159,13 +181,12 @@ def check_device_status(device=None) -> None:
     _status_watch.flush(device)
 
 
-def _report(ws: Optional[torch.Tensor], label: str, device) -> None:
-    """What follows a launch: the status word of a caller's workspace is watched; in debug mode every call is
-    synchronised and checked at once."""
-    if ws is not None:
-        _status_watch.watch(ws, label)
+def _status(lib, ws, label: str, stream_handle) -> None:
+    """What follows a launch with a workspace: its status word is watched, or in debug mode read at once."""
     if debug_device_status:
-        _status_watch.flush(device)
+        _abi.check(f"{label} (device)", lib.sa_read_status(_ptr(ws), ctypes.c_void_p(stream_handle)))
+    else:
+        _status_watch.watch(ws, label, stream_handle)
 
 
 def two_simplicial_attn_fwd_kernel(q, k1, k2, v1, v2, w1, w2, scale, k2_bias=0.0, v2_bias=0.0, halo1=0, halo2=0,
@@ -173,16 +194,28 @@ def two_simplicial_attn_fwd_kernel(q, k1, k2, v1, v2, w1, w2, scale, k2_bias=0.0
     """Forward launch (the reference's kernel of the same name, `simplicial/kernels.py:11-171`).
     Returns (O, LSE) with LSE = log sum exp of the logits, fp32 [B, H, N] (the reference's `M`)."""
     algo = algo or default_algo
-    ws = None
-    if _workspace is not _default_workspace:
-        p = _make_params(q, k1, k2, v1, v2, q, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo)
-        ws = _workspace(_abi.load().sa_forward_workspace_size(ctypes.byref(p)), q.device)
     if _status_watch.active:
         _status_watch.poll(q.device)
-    out = _abi.binding().forward(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo], ws)
-    if ws is not None or debug_device_status:
-        _report(ws, "sa_forward", q.device)
-    return out
+    if _workspace is _default_workspace:
+        out = _abi.binding().forward(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo])
+        if out is not None:
+            if debug_device_status:
+                _status_watch.flush(q.device)
+            return out
+    lib = _abi.load()
+    q, k1, k2, v1, v2 = (_unit_inner(t) for t in (q, k1, k2, v1, v2))
+    _check_inputs(q, k1, k2, v1, v2, halo1, halo2)
+    with torch.cuda.device(q.device):
+        o = torch.empty_like(q)                                   # triton_impl.py:23
+        lse = torch.empty((q.shape[0], q.shape[2], q.shape[1]), device=q.device, dtype=torch.float32)
+        p = _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo)
+        ws = _workspace(lib.sa_forward_workspace_size(ctypes.byref(p)), q.device)
+        sh = torch.cuda.current_stream().cuda_stream
+        rc = lib.sa_forward(ctypes.byref(p), _ptr(q), _ptr(k1), _ptr(k2), _ptr(v1), _ptr(v2), _ptr(o), _ptr(lse), _ptr(ws),
+                            ws.numel(), ctypes.c_void_p(sh))
+        _abi.check("sa_forward", rc)
+        _status(lib, ws, "sa_forward", sh)
+    return o, lse
 
 
 def two_simplicial_attn_bwd(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias=0.0, v2_bias=0.0, halo1=0, halo2=0,
@@ -191,20 +224,31 @@ def two_simplicial_attn_bwd(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bi
     two_simplicial_attn_bwd_kv2_kernel, `simplicial/kernels.py:175-571`).  Returns
     (dq, dk1, dk2, dv1, dv2), `None` where `need[i]` is false."""
     algo = algo or default_algo
-    ws = None
-    if _workspace is not _default_workspace:
-        p = _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo)
-        p.d_o = _strides(d_o)
-        p.dq, p.dk1, p.dk2, p.dv1, p.dv2 = (_strides(t) for t in (q, k1, k2, v1, v2))
-        ws = _workspace(_abi.load().sa_backward_workspace_size(ctypes.byref(p)), q.device)
     if _status_watch.active:
         _status_watch.poll(q.device)
-    bits = sum(1 << i for i, n in enumerate(need) if n)
-    grads = _abi.binding().backward(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo],
-                                    bits, ws)
-    if ws is not None or debug_device_status:
-        _report(ws, "sa_backward", q.device)
-    return grads
+    if _workspace is _default_workspace:
+        bits = sum(1 << i for i, n in enumerate(need) if n)
+        grads = _abi.binding().backward(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo],
+                                        bits)
+        if grads is not None:
+            if debug_device_status:
+                _status_watch.flush(q.device)
+            return grads
+    lib = _abi.load()
+    q, k1, k2, v1, v2, o, d_o = (_unit_inner(t) for t in (q, k1, k2, v1, v2, o, d_o))
+    _check_inputs(q, k1, k2, v1, v2, halo1, halo2)
+    with torch.cuda.device(q.device):
+        grads = [torch.empty_like(t) if n else None for t, n in zip((q, k1, k2, v1, v2), need)]
+        p = _make_params(q, k1, k2, v1, v2, o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, algo)
+        p.d_o = _strides(d_o)
+        p.dq, p.dk1, p.dk2, p.dv1, p.dv2 = (_strides(g) for g in grads)
+        ws = _workspace(lib.sa_backward_workspace_size(ctypes.byref(p)), q.device)
+        sh = torch.cuda.current_stream().cuda_stream
+        rc = lib.sa_backward(ctypes.byref(p), _ptr(q), _ptr(k1), _ptr(k2), _ptr(v1), _ptr(v2), _ptr(o), _ptr(lse), _ptr(d_o),
+                             *[_ptr(g) for g in grads], _ptr(ws), ws.numel(), ctypes.c_void_p(sh))
+        _abi.check("sa_backward", rc)
+        _status(lib, ws, "sa_backward", sh)
+    return tuple(grads)
 
 
 # When true every call synchronises and raises at once if a device-side bounded wait gave up; otherwise
@@ -254,11 +298,15 @@ class TwoSimplicialAttentionFunction(torch.autograd.Function):
 
 
 def _attend(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1=0, halo2=0):
-    """The operator with its autograd history: the binding's native node, or, where every call has to be checked or
-    given a caller's buffers, `TwoSimplicialAttentionFunction`."""
-    if debug_device_status or _status_watch.active or _workspace is not _default_workspace:
-        return TwoSimplicialAttentionFunction.apply(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2)
-    return _abi.binding().attention(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[default_algo])
+    """The operator with its autograd history: the binding's native node for a plain call, or
+    `TwoSimplicialAttentionFunction`, which traces, transforms and tensor subclasses know how to treat."""
+    if _workspace is _default_workspace and not debug_device_status:
+        if _status_watch.active:
+            _status_watch.poll(q.device)
+        o = _abi.binding().attention(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[default_algo])
+        if o is not None:
+            return o
+    return TwoSimplicialAttentionFunction.apply(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2)
 
 
 def two_simplicial_attention(q, k1, k2, v1, v2, w1, w2, scale=None, k2_bias=0.0, v2_bias=0.0, halo1=0, halo2=0):
