@@ -42,9 +42,9 @@ struct Config {
     int algo;
 };
 
-// ---- status words: pinned host memory, one 64-byte line per device and direction ({code, wait site, block, 0})
+// ---- status words: pinned host memory, 256 bytes per device and direction ({code, wait site, block, 0})
 constexpr int kMaxDevices = 64;
-constexpr int kSlotInts = 16;
+constexpr int kSlotInts = 64;
 enum Direction { kForward = 0, kBackward = 1 };
 const char* const kLabel[2] = {"sa_forward", "sa_backward"};
 
@@ -83,13 +83,14 @@ PyObject* g_on_error = nullptr;       // Python callable (function name, status,
     throw python_error(std::move(e));
 }
 
-// Raises if a kernel of an earlier call on the device gave up on a bounded wait; each report is given once.
+// Raises if a kernel of an earlier call on the device gave up on a bounded wait, and clears the word.  (While that kernel
+// still runs, another of its blocks may give up and leave a second report.)
 void poll_device(int device) {
     g_devices.fetch_or(1ull << device, std::memory_order_relaxed);
     for (Direction d : {kForward, kBackward}) {
         volatile int* s = slot(device, d);
         if (s[0] != 0) {
-            const int code = s[0], where = s[1], block = s[2];
+            const int code = s[0], where = s[1], block = s[2];      // (the device writes the code last)
             s[0] = s[1] = s[2] = 0;
             char text[96];
             snprintf(text, sizeof(text), "device side: wait site %d, block %d", where, block);
@@ -380,6 +381,16 @@ PyObject* py_poll(PyObject*, PyObject* device) {
     END_HANDLE_TH_ERRORS
 }
 
+// device, direction (0: forward, 1: backward)
+PyObject* py_status_word(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    expect(n, 2);
+    const int64_t device = int_arg(a[0]), direction = int_arg(a[1]);
+    TORCH_CHECK_INDEX(device >= 0 && device < kMaxDevices && (direction == kForward || direction == kBackward), "no such status word");
+    return PyLong_FromVoidPtr(status_word((int)device, (Direction)direction));
+    END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_devices(PyObject*, PyObject*) {
     const uint64_t bits = g_devices.load();
     PyObject* l = PyList_New(0);
@@ -404,6 +415,7 @@ PyMethodDef kMethods[] = {
     {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "(O, LSE); None for tensor subclasses"},
     {"backward", (PyCFunction)(void*)py_backward, METH_FASTCALL, "(dq, dk1, dk2, dv1, dv2); None for tensor subclasses"},
     {"poll", py_poll, METH_O, "raises if an earlier call on the device left a status"},
+    {"status_word", (PyCFunction)(void*)py_status_word, METH_FASTCALL, "address of the word that calls of a device and direction report to"},
     {"devices", py_devices, METH_NOARGS, "indices of the devices that have been called on"},
     {"on_error", py_on_error, METH_O, "sets the callable that raises for a status"},
     {nullptr, nullptr, 0, nullptr}};

@@ -29,7 +29,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
 // Status word of a call: in the first bytes of the caller's workspace, or wherever the caller asked for it
-// (device memory or pinned host memory; 16-byte aligned, written with one store).
+// (device memory or pinned host memory; 16-byte aligned, code and where written last and together).
 struct alignas(16) DeviceStatus {
     int code;        // 0 or SA_ERR_DEVICE_TIMEOUT
     int where;       // id of the wait that gave up

@@ -180,12 +180,15 @@ __device__ __forceinline__ bool mbar_wait_on(Test test, Probe probe, const WaitC
             if (t0 == 0) t0 = now;
             else if (now - t0 > ctx.limit_ns) {
                 asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(ctx.abort_flag), "r"(1u) : "memory");
-                // One 16-byte store, so that a reader never sees half a report; of several blocks that give up at the
-                // same time the last one stays (the word may be host memory, where the first could not be kept with
-                // an atomic operation on every system).
-                if (*(volatile int*)&ctx.status->code == 0)
-                    *reinterpret_cast<int4*>(ctx.status) = make_int4((int)SA_ERR_DEVICE_TIMEOUT, where, (int)blockIdx.x, 0);
-                __threadfence_system();
+                // Code and wait site in one 8-byte store behind the block, so that a reader that looks at the code first
+                // never sees half a report.  Of several blocks that give up at the same time one stays, perhaps with
+                // another one's block (the word may be host memory, where the first could not be kept with an atomic
+                // operation on every system).
+                if (*(volatile int*)&ctx.status->code == 0) {
+                    *(volatile int*)&ctx.status->block = (int)blockIdx.x;
+                    __threadfence_system();
+                    *reinterpret_cast<volatile uint64_t*>(ctx.status) = (uint64_t)(uint32_t)where << 32 | (uint32_t)SA_ERR_DEVICE_TIMEOUT;
+                }
                 return done(false);
             }
         }

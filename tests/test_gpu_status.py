@@ -64,6 +64,25 @@ def test_python_layer_reports_a_timeout_left_by_an_earlier_call():
     sab.check_device_status()                                                             # reported once
 
 
+@pytest.mark.parametrize("direction,label", [(0, "sa_forward"), (1, "sa_backward")])
+def test_report_in_the_pinned_word_is_raised_once(direction, label):
+    """The word that the binding's own calls report to: what a kernel leaves there is raised by the next forward call,
+    by the next backward (from autograd's thread) or by `check_device_status()`, and by one of them only."""
+    lib = _abi.load()
+    word = ctypes.c_void_p(_abi.binding().status_word(torch.cuda.current_device(), direction))
+    ts = [torch.randn(1, 64, 1, 64, device="cuda", dtype=torch.bfloat16).requires_grad_() for _ in range(5)]
+    call = lambda: sab.two_simplicial_attention(*ts, 16, 16)
+    o = call()
+    for ask in (call, lambda: torch.autograd.grad(o, ts, torch.ones_like(o), retain_graph=True), sab.check_device_status):
+        assert lib.sa_selftest_wait_timeout(word, 2_000_000, _stream()) == _abi.SA_OK
+        torch.cuda.synchronize()
+        with pytest.raises(_abi.SimplicialAttnError) as e:
+            ask()
+        assert e.value.status == _abi.SA_ERR_DEVICE_TIMEOUT and label in str(e.value) and "wait site 90, block 0" in str(e.value)
+        ask()
+    assert torch.equal(call(), o)
+
+
 def test_wait_limit_setter_keeps_results():
     """A shorter (still generous) limit for the real kernels changes nothing about their results."""
     lib = _abi.load()
