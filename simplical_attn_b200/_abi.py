@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 
 from . import build as _build
 
@@ -92,26 +93,36 @@ def load():
     return lib
 
 
-_binding = None
+_binding = None                  # not looked for yet; False: there is none
 
 
 def binding():
-    """The torch binding (`binding/sa_torch.cpp`): the operator on tensors as one native call per direction."""
+    """The torch binding (`binding/sa_torch.cpp`): the operator on tensors as one native call per direction.  None, after
+    a warning, where it is not built for this torch and cannot be built: the Python layer then calls the library through
+    ctypes (the same kernels; a small problem pays for its Python)."""
     global _binding
     if _binding is None:
         load()                                 # the binding links against the library
-        path = _build.BINDING
-        if _build.have_host_compiler():
-            path = _build.build_binding()
-        elif not os.path.exists(path):
-            raise OSError(f"{path} is missing and there is no C++ compiler to build it")
-        import importlib.util
-        spec = importlib.util.spec_from_file_location("sa_torch", path)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        mod.on_error(_raise)
-        _binding = mod
-    return _binding
+        try:
+            if _build.binding_stale():
+                if not _build.have_host_compiler():
+                    raise OSError(f"{_build.BINDING} was not built from these sources for this torch and this Python, and there is "
+                                  f"no C++ compiler")
+                _build.build_binding()
+            _binding = _import(_build.BINDING)
+        except (OSError, RuntimeError, ImportError) as e:
+            warnings.warn(f"calls go through ctypes, the native binding is not available: {e}", RuntimeWarning, stacklevel=3)
+            _binding = False
+    return _binding or None
+
+
+def _import(path: str):
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("sa_torch", path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.on_error(_raise)
+    return mod
 
 
 def _raise(fn: str, status: int, detail):

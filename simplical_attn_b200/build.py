@@ -5,6 +5,8 @@
 from __future__ import annotations
 
 import concurrent.futures
+import contextlib
+import fcntl
 import hashlib
 import os
 import shutil
@@ -122,28 +124,69 @@ def binding_digest() -> str:
     return h.hexdigest()
 
 
+def binding_stale() -> bool:
+    """Whether the binding is missing or was built from other sources, for another torch or another Python."""
+    if not os.path.exists(BINDING) or not os.path.exists(BINDING_STAMP):
+        return True
+    with open(BINDING_STAMP) as f:
+        return f.read().strip() != binding_digest()
+
+
+@contextlib.contextmanager
+def _locked():
+    os.makedirs(LIB_DIR, exist_ok=True)
+    with open(os.path.join(LIB_DIR, ".lock"), "w") as f:
+        fcntl.flock(f, fcntl.LOCK_EX)          # released when the file is closed
+        yield
+
+
 def build_binding(force: bool = False) -> str:
-    """Compile the torch binding if it is missing or was built from other sources (or for another torch)."""
-    digest = binding_digest()
-    if not force and os.path.exists(BINDING) and os.path.exists(BINDING_STAMP):
-        with open(BINDING_STAMP) as f:
-            if f.read().strip() == digest:
-                return BINDING
+    """Compile the torch binding if it is stale.  One process builds, the others wait for it; the file and its stamp
+    are put in place whole, so that a process that does not build never sees half of one."""
+    if not force and not binding_stale():
+        return BINDING
+    with _locked():
+        if force or binding_stale():
+            _compile_binding()
+    return BINDING
+
+
+def _put(path: str, write) -> None:
+    """Has `write` make a file beside `path`, then moves it there."""
+    part = f"{path}.{os.getpid()}.part"
+    try:
+        write(part)
+        os.replace(part, path)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
+
+
+def _write_text(text: str):
+    def write(path):
+        with open(path, "w") as f:
+            f.write(text)
+    return write
+
+
+def _compile_binding() -> None:
     import torch
     root = os.path.dirname(torch.__file__)
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), CUDA_INCLUDE,
            sysconfig.get_paths()["include"]]
     cmd = ([cxx_path()] + CXX_FLAGS + [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-I" + d for d in inc]
-           + ["-o", BINDING, BINDING_SRC, LIB, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           + [BINDING_SRC, LIB, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
               "-ltorch_python", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
-    os.makedirs(LIB_DIR, exist_ok=True)
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("the C++ compiler failed building " + BINDING)
-    with open(BINDING_STAMP, "w") as f:
-        f.write(digest + "\n")
-    return BINDING
+
+    def compile_to(path):
+        res = subprocess.run(cmd + ["-o", path], capture_output=True, text=True)
+        if res.returncode != 0:
+            sys.stderr.write(res.stdout + res.stderr)
+            raise RuntimeError("the C++ compiler failed building " + BINDING)
+
+    digest = binding_digest()
+    _put(BINDING, compile_to)
+    _put(BINDING_STAMP, _write_text(digest + "\n"))
 
 
 if __name__ == "__main__":

@@ -84,6 +84,11 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
 _default_workspace = _workspace       # where `_workspace` is replaced its buffers are used, and the binding is not
 
 
+def _native():
+    """The native binding, if it is there and buffers come from the default allocation."""
+    return _abi.binding() if _workspace is _default_workspace else None
+
+
 class _StatusWatch:
     """Surfaces device-side timeouts without a synchronisation per call.
 
@@ -165,7 +170,7 @@ class _StatusWatch:
         for index in indices:
             self.poll(torch.device("cuda", index), wait=True)
         binding = _abi.binding()
-        for index in binding.devices():
+        for index in binding.devices() if binding is not None else ():
             if device is None or index in indices:
                 torch.cuda.synchronize(index)
                 binding.poll(index)
@@ -196,8 +201,9 @@ def two_simplicial_attn_fwd_kernel(q, k1, k2, v1, v2, w1, w2, scale, k2_bias=0.0
     algo = algo or default_algo
     if _status_watch.active:
         _status_watch.poll(q.device)
-    if _workspace is _default_workspace:
-        out = _abi.binding().forward(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo])
+    native = _native()
+    if native is not None:
+        out = native.forward(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo])
         if out is not None:
             if debug_device_status:
                 _status_watch.flush(q.device)
@@ -226,10 +232,10 @@ def two_simplicial_attn_bwd(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bi
     algo = algo or default_algo
     if _status_watch.active:
         _status_watch.poll(q.device)
-    if _workspace is _default_workspace:
+    native = _native()
+    if native is not None:
         bits = sum(1 << i for i, n in enumerate(need) if n)
-        grads = _abi.binding().backward(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo],
-                                        bits)
+        grads = native.backward(q, k1, k2, v1, v2, o, lse, d_o, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[algo], bits)
         if grads is not None:
             if debug_device_status:
                 _status_watch.flush(q.device)
@@ -300,10 +306,11 @@ class TwoSimplicialAttentionFunction(torch.autograd.Function):
 def _attend(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1=0, halo2=0):
     """The operator with its autograd history: the binding's native node for a plain call, or
     `TwoSimplicialAttentionFunction`, which traces, transforms and tensor subclasses know how to treat."""
-    if _workspace is _default_workspace and not debug_device_status:
+    native = None if debug_device_status else _native()
+    if native is not None:
         if _status_watch.active:
             _status_watch.poll(q.device)
-        o = _abi.binding().attention(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[default_algo])
+        o = native.attention(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2, _ALGOS[default_algo])
         if o is not None:
             return o
     return TwoSimplicialAttentionFunction.apply(q, k1, k2, v1, v2, w1, w2, scale, k2_bias, v2_bias, halo1, halo2)

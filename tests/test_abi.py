@@ -1,6 +1,7 @@
 """CPU-side checks of the C-ABI library: it loads, exports every symbol the header declares, and
 its argument validation and kernel selection work without a GPU (no compute is launched)."""
 import ctypes
+import multiprocessing
 import os
 import re
 
@@ -113,6 +114,53 @@ def test_cpu_list_parsing_and_numa_helper_without_a_gpu():
     assert hp.local_cpus("cuda:0") is None or isinstance(hp.local_cpus("cuda:0"), set)      # no GPU here: None
     with hp.near("cuda:0") as took_effect:                                                   # must be harmless
         assert took_effect in (False, True)
+
+
+def test_binding_without_a_compiler(monkeypatch):
+    """A binding that was built for another torch (or not at all) is not loaded where it cannot be built again: calls go
+    through ctypes, after a warning."""
+    import torch
+    import simplical_attn_b200 as sab
+    from simplical_attn_b200 import build as b
+    assert _abi.binding() is not None and not b.binding_stale()
+    x = torch.zeros(1, 8, 1, 16)
+    for change in (lambda m: m.setattr(torch, "__version__", "0.0"), lambda m: m.setattr(b, "BINDING", b.BINDING + ".missing")):
+        with monkeypatch.context() as m:
+            m.setattr(_abi, "_binding", None)
+            m.setattr(b, "have_host_compiler", lambda: False)
+            change(m)
+            assert b.binding_stale()
+            with pytest.warns(RuntimeWarning, match="no C\\+\\+ compiler"):
+                assert _abi.binding() is None
+            with pytest.raises(RuntimeError, match="CUDA tensors only"):      # (this layer's check of the call)
+                sab.two_simplicial_attention(x, x, x, x, x, 4, 4)
+    assert _abi.binding() is not None
+
+
+def _rebuild(path):
+    from simplical_attn_b200 import build as b
+    _abi.load()                        # (what the binding is linked against)
+    b.LIB_DIR, b.BINDING, b.BINDING_STAMP = path, os.path.join(path, "sa_torch.so"), os.path.join(path, "sa_torch.so.sources")
+    b.build_binding()
+    return _abi._import(b.BINDING).devices()
+
+
+def test_binding_is_built_once_by_processes_that_start_together(tmp_path, monkeypatch):
+    """Several processes find the binding missing (the ranks of a job on a machine with another torch): one builds it, and
+    every one of them loads a whole file.  The compiler here copies the built one in two halves, with a pause, and counts."""
+    from simplical_attn_b200 import build as b
+    cxx = tmp_path / "g++"
+    cxx.write_text(f"""#!/bin/sh
+echo run >> {tmp_path}/runs
+while [ "$1" != -o ]; do shift; done
+head -c 100000 {b.BINDING} > "$2"; sleep 0.5; tail -c +100001 {b.BINDING} >> "$2"
+""")
+    cxx.chmod(0o755)
+    monkeypatch.setenv("PATH", f"{tmp_path}:{os.environ['PATH']}")
+    with multiprocessing.get_context("spawn").Pool(3) as pool:
+        assert pool.map(_rebuild, [str(tmp_path / "lib")] * 3, chunksize=1) == [[]] * 3
+    assert (tmp_path / "runs").read_text() == "run\n"
+    assert sorted(os.listdir(tmp_path / "lib")) == [".lock", "sa_torch.so", "sa_torch.so.sources"]
 
 
 def test_library_staleness_follows_source_contents(tmp_path, monkeypatch):

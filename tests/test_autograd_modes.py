@@ -86,6 +86,17 @@ def test_tensor_subclasses_are_kept():
 
 
 @pytest.mark.gpu
+def test_calls_without_the_binding(monkeypatch):
+    m, ts = sab.TwoSimplicialAttention(64, 50, 24), _inputs("cuda", grad=True)
+    want = m(*ts)
+    want_g = torch.autograd.grad(want, ts, torch.ones_like(want))
+    monkeypatch.setattr(_abi, "_binding", False)
+    o = m(*ts)
+    assert torch.equal(o, want) and all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(o, ts, torch.ones_like(o)), want_g))
+    sab.check_device_status()
+
+
+@pytest.mark.gpu
 def test_saved_tensor_hooks_and_checkpointing():
     from torch.utils.checkpoint import checkpoint
     m, ts = sab.TwoSimplicialAttention(64, 50, 24), _inputs("cuda", grad=True)
