@@ -166,6 +166,11 @@ int sa_selftest_wait_timeout(void* workspace, uint64_t limit_ns, void* stream);
  * sa_status if `p` is invalid. */
 int sa_resolve_algo(const sa_params* p);
 
+/* How the general kernels would make the call: bit 0 for the forward, 1 for dQ, 2 for dK1 / dV1, 3 for dK2 / dV2, set where
+ * a warp per output row is expected to be faster than tiles (short windows or sequences), or -sa_status.  The choice
+ * changes the order of the sums, nothing else.  No counterpart in the reference. */
+int sa_general_plan(const sa_params* p);
+
 /* Strided copy between host and device (either direction, or device to device) on `stream`: `rows`
  * pieces of `row_bytes` bytes, `src_pitch` / `dst_pitch` bytes apart.  Used to move one group of
  * heads of a [B, N, H, D] tensor that lives in pinned host memory without staging it first.  Host

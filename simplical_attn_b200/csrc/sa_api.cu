@@ -472,6 +472,15 @@ int sa_resolve_algo(const sa_params* p) {
     return resolve(p, true);
 }
 
+int sa_general_plan(const sa_params* p) {
+    const int v = validate(p);
+    if (v != SA_OK) return -v;
+    const KParams k = make_kparams(p);
+    int bits = 0;
+    for (int i = 0; i < 4; ++i) bits |= sa::general::by_rows((sa::general::Kernel)i, k, plan_sm_count()) ? 1 << i : 0;
+    return bits;
+}
+
 size_t sa_forward_workspace_size(const sa_params* p) {
     if (validate(p) != SA_OK || resolve(p, false) != SA_ALGO_TCGEN05) return kStatusBytes;
     const KParams k = make_kparams(p);

@@ -12,9 +12,9 @@
 // C = dO_i * (V2_k + bias) against tiles of K1/V1 rows, all in shared memory as fp32; a thread holds 4 rows by up to 4
 // columns of the score tile and 4 rows by D/16 columns of the accumulators, so an operand read from shared memory is
 // used four times.  Large problems are bound by the FMA pipes and shared-memory reads at about equal shares, small ones
-// by the latency of a block's chain of loads.  (One warp per output row with the head dim across its lanes, as
-// before, spent five to ten shuffles in a serial chain on every (j, k) pair: all kernels of a forward and backward
-// together 846 -> 141 us for fp32 B1 N256 H2 D64 w 64/16, 1448 -> 463 us for bf16 B2 N512 H4 D32 w 32/32.)
+// by the latency of a block's chain of loads.  All kernels of a forward and backward together take 141 us for fp32
+// B1 N256 H2 D64 w 64/16 and 463 us for bf16 B2 N512 H4 D32 w 32/32; by a warp per output row (sa_general_rows.cuh) 846 and
+// 1448 us.  Short windows, which would leave most of a tile empty, go there.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "sa_common.cuh"
+#include "sa_general_rows.cuh"
 
 namespace sa {
 namespace general {
@@ -605,9 +606,71 @@ inline int owners_per_block(const KParams& p, long n_own, long heads, int sm_cou
     return n;
 }
 
+// Blocks of a cluster of the dK1/dV1 kernel: enough of them for every multiprocessor, as long as each has tiles to work on.
+inline long col_tiles(const KParams& p) {
+    return ((long)p.G * (p.w1 + kColRows < p.N ? p.w1 + kColRows : p.N) * p.w2 + kRows - 1) / kRows;
+}
+inline int col_cluster(const KParams& p, int sm_count) {
+    const long items = (long)p.B * p.Hkv * ((p.n1 + kColRows - 1) / kColRows), tiles = col_tiles(p);
+    int nrank = 1;
+    while (nrank < 8 && items * nrank * 2 <= 2L * sm_count && nrank * 2 <= tiles) nrank *= 2;
+    return nrank;
+}
+
+// Tiles or a warp per output row: the smaller of two estimates, in us, with constants measured on a B200 over 437 problems
+// (head dims 32, 64, 128, 256, windows 1 ... 1024 / 1 ... 160, sequences of 1 ... 4096 rows): the faster of the two kernels within
+// 5 % in 95 % of them, at worst 0.53 of its speed (a few short launches).
+//   rows:  0.14 R + (pairs + outer o) max(0.32, pair R), with R output rows (warps) per multiprocessor, a row's (j, k) pairs
+//          and outer steps (K2 rows, or for dK1/dV1 queries);
+//   tiles: max(1.75, blocks per multiprocessor) x (passes x (tile + group x 16-column groups)), for dK1/dV1
+//          (tile + group x tiles).
+enum Kernel { kFwd = 0, kDq = 1, kKv1 = 2, kKv2 = 3 };
+struct Cost {
+    double pair[4], o, tile[4], group[4];      // by padded head dim 32, 64, 128, 256
+};
+constexpr Cost kCost[4] = {
+    {{.013, .013, .019, .028}, .5, {3.8, 5.4, 18, 25}, {.97, 1.4, 2.6, 6.8}},
+    {{.013, .013, .017, .031}, .68, {3.5, 6.6, 20, 34}, {1.3, 1.8, 3.5, 9.2}},
+    {{.013, .014, .021, .086}, 1.2, {2.5, 2.5, 0, 0}, {4.8, 8.1, 21, 45}},
+    {{.013, .015, .020, .039}, 1.5, {3.6, 11, 21, 37}, {1.5, 2.7, 4.6, 12}},
+};
+
+// K1 (K2) rows that a query sees, averaged over the queries: windows are cut at the first row that exists.
+inline double mean_window(const KParams& p, int w, int halo) {
+    const double n = p.N, cut = w - halo < 0 ? 0 : w - halo < p.N ? w - halo : p.N;
+    return (cut * (cut + 1) / 2 + cut * halo + (n - cut) * w) / n;
+}
+
+inline bool by_rows(Kernel kernel, const KParams& p, int sm_count) {
+    const Cost& c = kCost[kernel];
+    const int d = p.D <= 32 ? 0 : p.D <= 64 ? 1 : p.D <= 128 ? 2 : 3;
+    const int n_out = kernel == kKv1 ? p.n1 : kernel == kKv2 ? p.n2 : p.N;
+    const double heads = kernel < kKv1 ? p.H : p.Hkv, group = kernel < kKv1 ? 1 : p.G;
+    const double m1 = mean_window(p, p.w1, p.halo1), m2 = mean_window(p, p.w2, p.halo2), per = group * p.N / n_out;
+    const double warps = p.B * heads * n_out / sm_count;
+    const double rows = .14 * warps + per * (m1 * m2 + c.o * (kernel == kKv1 ? m1 : m2)) * fmax(.32, c.pair[d] * warps);
+    double blocks, tiles;
+    if (kernel == kKv1) {
+        const int nrank = col_cluster(p, sm_count);
+        blocks = p.B * heads * ((n_out + kColRows - 1) / kColRows) * nrank;
+        tiles = c.tile[d] + c.group[d] * ((col_tiles(p) + nrank - 1) / nrank);
+    } else {
+        const int owners = owners_per_block(p, n_out, (long)heads, sm_count);
+        const long span = p.w1 + (kernel == kKv2 ? owners + (p.w2 < kRows ? p.w2 : kRows) - 2 : owners - 1);
+        blocks = p.B * heads * ((n_out + owners - 1) / owners);
+        tiles = group * ((p.w2 + kRows - 1) / kRows) * (c.tile[d] + c.group[d] * (((span < p.n1 ? span : p.n1) + 15) / 16));
+    }
+    return rows <= fmax(1.75, blocks / sm_count) * tiles;
+}
+
 template <typename T, int DP>
 cudaError_t launch_fwd_t(const KParams& p, const void* q, const void* k1, const void* k2, const void* v1,
                          const void* v2, void* o, float* lse, int sm_count, cudaStream_t st) {
+    if (by_rows(kFwd, p, sm_count)) {
+        row_fwd_kernel<T, DP / 32><<<row_blocks((long)p.B * p.H * p.N), kWarpsPerBlock * 32, 0, st>>>(p, (const T*)q, (const T*)k1, (const T*)k2,
+                                                                                                      (const T*)v1, (const T*)v2, (T*)o, lse);
+        return cudaGetLastError();
+    }
     const int owners = owners_per_block(p, p.N, p.H, sm_count);
     const long blocks = (long)p.B * p.H * ((p.N + owners - 1) / owners);
     if (!allow_dynamic_smem((const void*)fwd_kernel<T, DP>, Shape<DP>::kFwdBytes)) return cudaErrorInvalidValue;
@@ -621,7 +684,10 @@ cudaError_t launch_bwd_t(const KParams& p, const void* q, const void* k1, const 
                          const void* v2, const void* o, const float* lse, const void* d_o, void* dq, void* dk1,
                          void* dk2, void* dv1, void* dv2, int sm_count, cudaStream_t st) {
     using S = Shape<DP>;
-    if (dq) {
+    if (dq && by_rows(kDq, p, sm_count)) {
+        row_dq_kernel<T, DP / 32><<<row_blocks((long)p.B * p.H * p.N), kWarpsPerBlock * 32, 0, st>>>(
+            p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o, (T*)dq);
+    } else if (dq) {
         const int owners = owners_per_block(p, p.N, p.H, sm_count);
         auto kern = bwd_row_kernel<T, DP, false>;
         if (!allow_dynamic_smem((const void*)kern, S::kBwdBytes)) return cudaErrorInvalidValue;
@@ -629,14 +695,14 @@ cudaError_t launch_bwd_t(const KParams& p, const void* q, const void* k1, const 
             p, owners, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o, (T*)dq,
             (T*)nullptr, (T*)nullptr);
     }
-    if (dk1 || dv1) {
+    if ((dk1 || dv1) && by_rows(kKv1, p, sm_count)) {
+        row_kv1_kernel<T, DP / 32><<<row_blocks((long)p.B * p.Hkv * p.n1), kWarpsPerBlock * 32, 0, st>>>(
+            p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o, (T*)dk1, (T*)dv1);
+    } else if (dk1 || dv1) {
         auto kern = bwd_col_kernel<T, DP>;
         if (!allow_dynamic_smem((const void*)kern, S::kColBytes)) return cudaErrorInvalidValue;
         const long items = (long)p.B * p.Hkv * ((p.n1 + kColRows - 1) / kColRows);
-        // blocks per cluster: enough of them for every multiprocessor, as long as each has tiles to work on
-        const long tiles = ((long)p.G * (p.w1 + kColRows < p.N ? p.w1 + kColRows : p.N) * p.w2 + kRows - 1) / kRows;
-        int nrank = 1;
-        while (nrank < 8 && items * nrank * 2 <= 2L * sm_count && nrank * 2 <= tiles) nrank *= 2;
+        const int nrank = col_cluster(p, sm_count);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(items * nrank));
         cfg.blockDim = dim3(kThreads);
@@ -652,7 +718,10 @@ cudaError_t launch_bwd_t(const KParams& p, const void* q, const void* k1, const 
                                                  (const T*)o, lse, (const T*)d_o, (T*)dk1, (T*)dv1);
         if (e != cudaSuccess) return e;
     }
-    if (dk2 || dv2) {
+    if ((dk2 || dv2) && by_rows(kKv2, p, sm_count)) {
+        row_kv2_kernel<T, DP / 32><<<row_blocks((long)p.B * p.Hkv * p.n2), kWarpsPerBlock * 32, 0, st>>>(
+            p, (const T*)q, (const T*)k1, (const T*)k2, (const T*)v1, (const T*)v2, (const T*)o, lse, (const T*)d_o, (T*)dk2, (T*)dv2);
+    } else if (dk2 || dv2) {
         const int owners = owners_per_block(p, p.n2, p.Hkv, sm_count);
         auto kern = bwd_row_kernel<T, DP, true>;
         if (!allow_dynamic_smem((const void*)kern, S::kBwdBytes)) return cudaErrorInvalidValue;

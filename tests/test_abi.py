@@ -84,6 +84,21 @@ def test_kernel_selection():
     assert extra >= (4096 * 4 * 128 + 4 * 4096 * 2 * 128) * 2
 
 
+def test_general_kernels_take_short_windows_by_rows():
+    """Problems far from the line between the two kinds of general kernels, as measured: fp32, by rows and by tiles, us, forward
+    (479 / 1100 at w 16/33, 4314 / 1698 at w 64/64, 12 / 486 for 4096 sequences of one row)."""
+    lib = _abi.load()
+    plan = lambda **kw: lib.sa_general_plan(ctypes.byref(_params(dtype=_abi.SA_F32, Hkv=4, **kw)))
+    assert plan(B=4, N=512, D=128, w1=16, w2=33) == 15
+    assert plan(B=4, N=512, D=128, w1=64, w2=64) == 0
+    assert plan(B=4096, N=1, D=64, w1=64, w2=64) == 15
+    assert plan(B=4, N=512, D=256, w1=4, w2=100) == 15
+    assert plan(B=1, N=512, D=64, w1=512, w2=512) == 0
+    assert plan(B=4, N=512, D=32, w1=32, w2=33) == 0
+    assert plan(N=64, D=64, w1=4, w2=4, halo1=2**20, halo2=2**20) >= 0            # (no overflow)
+    assert plan(w1=0) == -2
+
+
 def test_python_layer_rejects_cpu_tensors():
     import torch
     import simplical_attn_b200 as sab

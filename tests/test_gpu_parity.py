@@ -5,6 +5,7 @@ Tolerances (stated by the target for bf16 kernels vs the fp32 reference on bf16-
 max-abs <= 2e-2 on O, relative L2 <= 1e-2 on each gradient.  fp32 tensors through the general
 kernels are held to 1e-4.
 """
+import ctypes
 import math
 
 import pytest
@@ -12,6 +13,7 @@ import torch
 
 import simplical_attn_b200 as sab
 from oracle import c_oracle, simplicial_oracle as so
+from simplical_attn_b200 import _abi
 from simplical_attn_b200 import simplicial_attn as host
 from tests import golden_util as gu
 
@@ -501,7 +503,25 @@ GENERAL_CASES = [
     (1, 200, 2, 1, 200, 80, 130, 0.0, 0.0, 0, 0),
     (1, 75, 1, 1, 256, 100, 7, 0.1, 0.0, 0, 0),
     (3, 600, 4, 4, 64, 128, 2, 0.0, 0.0, 0, 0),
+    (1, 160, 2, 1, 33, 90, 3, 0.1, -0.1, 0, 0),
+    (1, 140, 4, 2, 96, 100, 24, 0.0, 0.2, 99, 23),
+    (1, 190, 1, 1, 130, 120, 16, 0.0, 0.0, 0, 0),
+    (1, 150, 2, 1, 256, 150, 7, 0.1, 0.0, 0, 0),
+    (1, 130, 2, 2, 8, 100, 5, 0.0, 0.0, 3, 2),
+    (2, 70, 2, 1, 100, 6, 5, 0.0, 0.1, 0, 0),
+    (4, 40, 2, 2, 64, 3, 3, 0.1, 0.0, 2, 2),
 ]
+
+
+def test_general_cases_reach_both_kinds_of_general_kernels():
+    """Every kernel, by rows and by tiles, at every padded head dim."""
+    seen = set()
+    for B, N, H, Hkv, D, w1, w2, _, _, h1, h2 in GENERAL_CASES:
+        p = _abi.Params()
+        p.B, p.N, p.H, p.Hkv, p.D, p.w1, p.w2, p.halo1, p.halo2, p.dtype, p.scale = B, N, H, Hkv, D, w1, w2, h1, h2, _abi.SA_F32, 1.0
+        plan = _abi.load().sa_general_plan(ctypes.byref(p))
+        seen |= {(max(32, 1 << (D - 1).bit_length()), kernel, plan >> kernel & 1) for kernel in range(4)}
+    assert len(seen) == 4 * 4 * 2, sorted({(d, k, r) for d in (32, 64, 128, 256) for k in range(4) for r in (0, 1)} - seen)
 
 
 @pytest.mark.parametrize("case", GENERAL_CASES)
@@ -522,10 +542,11 @@ def test_general_kernels_vs_cpu_oracle_fp32(case):
             assert so.rel_l2(g.cpu().double(), r) <= 1e-5, nm
 
 
-def test_general_kernels_keep_values_that_are_not_finite_to_their_windows():
+@pytest.mark.parametrize("N,w1,w2", [(160, 40, 8), (300, 128, 8)])      # the second by tiles
+def test_general_kernels_keep_values_that_are_not_finite_to_their_windows(N, w1, w2):
     """An infinity in one row of an input reaches the results of the queries that see it, and of the rows that those
     see, and no others, although tiles hold rows of several windows: everything else equals the run on finite inputs."""
-    B, N, H, D, w1, w2 = 1, 160, 1, 32, 40, 8
+    B, H, D = 1, 1, 32
     ts = dict(zip(("q", "k1", "k2", "v1", "v2", "do"), so.make_inputs(B, N, H, H, D, seed=21, seed_do=22)))
     cfg = dict(w1=w1, w2=w2, scale=1.0 / math.sqrt(D), k2_bias=0.0, v2_bias=0.0)
     clean = _run(ts, cfg, "general", dtype=torch.float32)
