@@ -105,8 +105,13 @@ __device__ __forceinline__ void row_stats(float* delta, float* L, const int* ri,
     if (i >= 0) {
         const T* orow = o + head_of(r, 0) + (int64_t)i * os;
         const T* drow = d_o + head_of(r, 1) + (int64_t)i * dos;
-#pragma unroll 8
-        for (int d = part; d < D; d += 4) s = fmaf(to_f<T>(drow[d]), to_f<T>(orow[d]), s);
+        for (int d0 = part; d0 < D; d0 += 32) {          // (in blocks, as in `product`)
+            float t = 0.f;
+#pragma unroll
+            for (int d = d0; d < d0 + 32; d += 4)
+                if (d < D) t = fmaf(to_f<T>(drow[d]), to_f<T>(orow[d]), t);
+            s += t;
+        }
     }
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
@@ -116,7 +121,8 @@ __device__ __forceinline__ void row_stats(float* delta, float* L, const int* ri,
     }
 }
 
-// s[a][c] = X[4 ty + a] . Y[tx + 16 c]
+// s[a][c] = X[4 ty + a] . Y[tx + 16 c], summed in blocks of 16 products: a single chain over the head dim made the error of
+// dQ and dK2 against 64 bits larger than the row kernels' (fp32 D128 w 100/40: 6.6e-7 and 6.9e-7 against 5.6e-7 and 6.1e-7).
 template <int DP, int NC>
 __device__ __forceinline__ void product(const float* X, const float* Y, int ty, int tx, float (&s)[4][NC]) {
     constexpr int P = Shape<DP>::kPitch;
@@ -124,20 +130,28 @@ __device__ __forceinline__ void product(const float* X, const float* Y, int ty, 
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int c = 0; c < NC; ++c) s[a][c] = 0.f;
-#pragma unroll 4
-    for (int d = 0; d < DP; d += 4) {
-        float x[4][4];
+#pragma unroll 1
+    for (int d0 = 0; d0 < DP; d0 += 16) {
+        float t[4][NC];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) lds_vec<4>(X + (4 * ty + a) * P + d, x[a]);
+        for (int d = d0; d < d0 + 16; d += 4) {
+            float x[4][4];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            float y[4];
-            lds_vec<4>(Y + (tx + 16 * c) * P + d, y);
+            for (int a = 0; a < 4; ++a) lds_vec<4>(X + (4 * ty + a) * P + d, x[a]);
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int c = 0; c < NC; ++c) {
+                float y[4];
+                lds_vec<4>(Y + (tx + 16 * c) * P + d, y);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[a][c] = fmaf(x[a][e], y[e], s[a][c]);
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) t[a][c] = d == d0 && e == 0 ? x[a][e] * y[e] : fmaf(x[a][e], y[e], t[a][c]);
+            }
         }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) s[a][c] += t[a][c];
     }
 }
 

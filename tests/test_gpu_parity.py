@@ -542,6 +542,19 @@ def test_general_kernels_vs_cpu_oracle_fp32(case):
             assert so.rel_l2(g.cpu().double(), r) <= 1e-5, nm
 
 
+def test_general_kernels_fp32_error_at_wide_heads():
+    """The scores' dot products are summed in blocks.  In one chain over 256 products the error of dQ and dK2 against 64 bits
+    is 8e-7 here, by a warp with the head dim across its lanes (32 chains of 8, then a tree) 5.4e-7, in blocks of 16
+    4.2e-7: the bound is the second."""
+    N, D, w1, w2 = 300, 256, 120, 20
+    ts = so.make_inputs(1, N, 1, 1, D, seed=51, seed_do=52, bf16_round=False)
+    cfg = dict(w1=w1, w2=w2, scale=1.0 / math.sqrt(D), k2_bias=0.0, v2_bias=0.0)
+    _, _, grads = _run(dict(zip(("q", "k1", "k2", "v1", "v2", "do"), ts)), cfg, "general", dtype=torch.float32)
+    ref = so.forward_backward(*ts, w1, w2, cfg["scale"], dtype=torch.float64)
+    for nm, i in (("dq", 0), ("dk2", 2)):
+        assert so.rel_l2(grads[i].cpu().double(), ref[2 + i]) <= 5.4e-7, nm
+
+
 @pytest.mark.parametrize("N,w1,w2", [(160, 40, 8), (300, 128, 8)])      # the second by tiles
 def test_general_kernels_keep_values_that_are_not_finite_to_their_windows(N, w1, w2):
     """An infinity in one row of an input reaches the results of the queries that see it, and of the rows that those
