@@ -81,7 +81,8 @@ __device__ __forceinline__ bool load_rows(float* dst, const T* __restrict__ x, i
     return bad;
 }
 
-// The operand rows of a tile: dst[r] = x[ri[r]] * (y[rk[r]] + bias) * mult, zeros where ri[r] < 0.
+// The operand rows of a tile: dst[r] = (x[ri[r]] * mult) * (y[rk[r]] + bias), zeros where ri[r] < 0.  (In this order, as in
+// sa_general_rows.cuh: a scale that brings large inputs into range acts before they are multiplied with each other.)
 template <typename T, int DP>
 __device__ __forceinline__ void form_rows(float* dst, const int* ri, const int* rk, const T* __restrict__ x, int64_t xs,
                                           const T* __restrict__ y, int64_t ys, float bias, float mult, int D) {
@@ -89,7 +90,7 @@ __device__ __forceinline__ void form_rows(float* dst, const int* ri, const int* 
     for (int idx = threadIdx.x; idx < kRows * DP; idx += kThreads) {
         const int r = idx / DP, d = idx % DP;
         float v = 0.f;
-        if (ri[r] >= 0 && d < D) v = to_f<T>(x[(int64_t)ri[r] * xs + d]) * (to_f<T>(y[(int64_t)rk[r] * ys + d]) + bias) * mult;
+        if (ri[r] >= 0 && d < D) v = to_f<T>(x[(int64_t)ri[r] * xs + d]) * mult * (to_f<T>(y[(int64_t)rk[r] * ys + d]) + bias);
         dst[r * Shape<DP>::kPitch + d] = v;
     }
 }
@@ -528,7 +529,7 @@ bwd_col_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, con
             const int r = idx / DP, d = idx % DP, i = ri[r], h = rh[r];
             float a = 0.f, c = 0.f;
             if (i >= 0 && d < p.D) {
-                a = to_f<T>(q[b * p.q.b + h * p.q.h + (int64_t)i * p.q.n + d]) * (to_f<T>(k2h[(int64_t)rk[r] * p.k2.n + d]) + p.k2_bias) * p.scale;
+                a = to_f<T>(q[b * p.q.b + h * p.q.h + (int64_t)i * p.q.n + d]) * p.scale * (to_f<T>(k2h[(int64_t)rk[r] * p.k2.n + d]) + p.k2_bias);
                 c = to_f<T>(d_o[b * p.d_o.b + h * p.d_o.h + (int64_t)i * p.d_o.n + d]) * (to_f<T>(v2h[(int64_t)rk[r] * p.v2.n + d]) + p.v2_bias);
             }
             bad |= not_finite(a) || not_finite(c);

@@ -145,7 +145,7 @@ row_dq_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, cons
         load_row<T, EPL>(k2h + (long)k * p.k2.n, D, lane, k2v, p.k2_bias);
         load_row<T, EPL>(v2h + (long)k * p.v2.n, D, lane, c, p.v2_bias);
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) { a[e] = qv[e] * k2v[e] * p.scale; c[e] *= dov[e]; g[e] = 0.f; }
+        for (int e = 0; e < EPL; ++e) { a[e] = qv[e] * p.scale * k2v[e]; c[e] *= dov[e]; g[e] = 0.f; }
         for (int j = j_lo; j <= j_hi; ++j) {
             float k1v[EPL], v1v[EPL];
             load_row<T, EPL>(k1h + (long)j * p.k1.n, D, lane, k1v);
@@ -236,7 +236,7 @@ row_kv2_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, con
             load_query<T, EPL>(p, q, o, d_o, lse, b, h, i, lane, qv, dov, delta, L);
             float a[EPL], c[EPL], g[EPL], u[EPL];
 #pragma unroll
-            for (int e = 0; e < EPL; ++e) { a[e] = qv[e] * k2v[e] * p.scale; c[e] = dov[e] * v2v[e]; g[e] = 0.f; u[e] = 0.f; }
+            for (int e = 0; e < EPL; ++e) { a[e] = qv[e] * p.scale * k2v[e]; c[e] = dov[e] * v2v[e]; g[e] = 0.f; u[e] = 0.f; }
             const int j_hi = i + p.halo1, j_lo = max(0, j_hi - p.w1 + 1);
             for (int j = j_lo; j <= j_hi; ++j) {
                 float k1v[EPL], v1v[EPL];

@@ -542,6 +542,22 @@ def test_general_kernels_vs_cpu_oracle_fp32(case):
             assert so.rel_l2(g.cpu().double(), r) <= 1e-5, nm
 
 
+@pytest.mark.parametrize("w1,w2", [(3, 2), (128, 24)])                  # by rows, by tiles
+def test_general_kernels_apply_the_scale_before_large_inputs_meet(w1, w2):
+    """Q * 2^75 and K2 * 2^55 overflow fp32 together; with a scale of 2^-130 less they do not, and as powers of two are
+    exact, the results are those of the inputs as they were (dQ and dK2 but for their factors)."""
+    D = 32
+    ts = dict(zip(("q", "k1", "k2", "v1", "v2", "do"), so.make_inputs(1, 200, 1, 1, D, seed=53, seed_do=54)))
+    cfg = dict(w1=w1, w2=w2, scale=2.0 ** 6, k2_bias=0.0, v2_bias=0.0)
+    ts["q"] = ts["q"] * 2.0 ** -8
+    o, lse, g = _run(ts, cfg, "general", dtype=torch.float32)
+    big = dict(ts, q=ts["q"] * 2.0 ** 75, k2=ts["k2"] * 2.0 ** 55)
+    o2, lse2, g2 = _run(big, dict(cfg, scale=2.0 ** (6 - 130)), "general", dtype=torch.float32)
+    assert bool(torch.isfinite(o).all()) and torch.equal(o, o2) and torch.equal(lse, lse2)
+    for i in (1, 3, 4):
+        assert torch.equal(g[i], g2[i]), i
+
+
 def test_general_kernels_fp32_error_at_wide_heads():
     """The scores' dot products are summed in blocks.  In one chain over 256 products the error of dQ and dK2 against 64 bits
     is 8e-7 here, by a warp with the head dim across its lanes (32 chains of 8, then a tree) 5.4e-7, in blocks of 16
