@@ -34,6 +34,8 @@
 // both softmax groups split its columns and hand P^T, later dS^T, to the MMA warp in two parts.
 #pragma once
 
+#include <math.h>
+
 #include <type_traits>
 
 #include "sa_ptx.cuh"
@@ -1845,6 +1847,31 @@ inline BwdPlan bwd_plan(const KParams& k, int sm_count) {
 
 inline size_t bwd_workspace_bytes(const KParams& k, int sm_count) { return bwd_plan(k, sm_count).total; }
 
+// The row kernel needs nothing from the column kernel, so it can run beside it.  Where the column kernel's grid covers more
+// than half of the multiprocessors, the row kernel's blocks follow on those whose last column block has finished.  (Not
+// without a ring in shared memory, when it adds up dK2 and dV2 in device memory: B1 N2048 H8 D128 w 128/200, backward 15818 us
+// one after the other, 16588 so.)  Where it covers less, the row kernel can have a grid of the rest, so that no block waits
+// for a multiprocessor; that pays unless the row kernel is the longer one by far.  True if the longer of the two, side by
+// side, is estimated to be shorter than both, one after the other: us, from measured kernels, of a tile of the column
+// kernel and of a unit of the row kernel and its tiles; on fewer multiprocessors a unit takes a little less.
+// Backward, us, one after the other and side by side: B2 N512 H4 D64 w 32/32 (32 column blocks) 174 and 107; B1 N4096
+// H16/2 D128 w 512/32 4180 and 2345, but w 64/4 1167 and 1458, w 64/1 1674 and 2663, w 64/128 39160 and 57830; B1 N2048 H8/1
+// D128 w 512/128 26760 and 14020.
+inline bool side_by_side(const BwdTcParams& P, int qpt, int sm_count, long col_grid, bool ring) {
+    const KParams& k = P.k;
+    const int dw = 1 << P.dw_log2;
+    const bool wide = k.D > 64;
+    const double queries = k.w1 + 127 < k.N ? k.w1 + 127 : k.N, tiles = (k.w1 + qpt + 62) / 64;
+    const double col = (queries * dw / kColTileRows + 1) * k.G * (dw < 16 ? 4.8 : dw > 64 && wide ? 2.8 : 1.8);
+    double unit = tiles;
+    if (dw < 16) unit += (12 + 190 / pow(dw, 1.4)) * (wide ? 1.6 : 1);
+    else if (dw > 64) unit += ring ? 6.5 : 77;
+    else unit = (dw == 16 ? 7 : dw == 32 ? 4.6 : 5.2) * (wide ? 1.4 : 1) + tiles * (wide ? .6 : .35);
+    auto row = [&](long sms) { return (double)((P.num_row_items + sms - 1) / sms) * P.units_per_run * unit; };
+    const double beside = .93 * row(sm_count - col_grid);
+    return (beside > col ? beside : col) < col + row(sm_count);
+}
+
 typedef bool (*MakeMapFn)(CUtensorMap*, const void*, int, int, int, int, const sa_strides&, int, bool);
 
 // Returns an sa_status, or -1 when the tensor-core backward does not cover the problem.  F16: the tensors are
@@ -1905,12 +1932,6 @@ int launch_bwd_t(const KParams& k, const void* q, const void* k1, const void* k2
         CUtensorMap m1, m2;
         if (!make_map(&m1, k1, k.B, k.n1, k.Hkv, k.D, k.k1, kStreamRows, F16)) return SA_ERR_BAD_STRIDE;
         if (!make_map(&m2, v1, k.B, k.n1, k.Hkv, k.D, k.v1, kStreamRows, F16)) return SA_ERR_BAD_STRIDE;
-        // The row kernel needs nothing from the column kernel, so it is launched to run beside it: on the multiprocessors
-        // that a small problem's column kernel leaves idle (its grid is then no larger than that, so that no block has to
-        // wait for one), or on those whose last column block has finished.  B2 N512 H4 D64 w 32/32 (32 column blocks), forward
-        // and backward: 170 us one after the other, 114 us side by side.
-        const long sms = col_grid <= sm_count / 2 ? sm_count - col_grid : sm_count;
-        const long grid = P.num_row_items < sms ? P.num_row_items : sms;
         const int need_kv2 = (dk2 || dv2) ? 1 : 0;
         // shared-memory ring of fp32 dK2/dV2 rows beside the tiles: with the 3-stage K1/V1 ring if it fits,
         // else with 2 stages, else none (partials then accumulate in the workspace)
@@ -1921,6 +1942,16 @@ int launch_bwd_t(const KParams& k, const void* q, const void* k1, const void* k2
             if (!need_kv2 || smem > max_dyn) { ring_rows = 0; smem = k_ring + 1024 + extra; }
             if (smem < k_min) smem = k_min;
             if (!allow_dynamic_smem((const void*)kern, max_dyn)) return false;
+            const bool ring = ring_rows > 0 || !need_kv2;
+            bool beside = false;
+            long sms = sm_count;
+            if (col_grid > sm_count / 2) {
+                beside = ring;
+            } else if (col_grid > 0) {
+                beside = side_by_side(P, pl.qpt, sm_count, col_grid, ring);
+                if (beside) sms = sm_count - col_grid;
+            }
+            const long grid = P.num_row_items < sms ? P.num_row_items : sms;
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3((unsigned)grid);
             cfg.blockDim = dim3((unsigned)threads);
@@ -1930,7 +1961,7 @@ int launch_bwd_t(const KParams& k, const void* q, const void* k1, const void* k2
             attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr.val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = &attr;
-            cfg.numAttrs = col_grid > 0 ? 1 : 0;
+            cfg.numAttrs = beside ? 1 : 0;
             return cudaLaunchKernelEx(&cfg, kern, P, m1, m2, bf(q), bf(k2), bf(v2), bf(d_o), (__nv_bfloat16*)dq, need_kv2, ring_rows) ==
                    cudaSuccess;
         };

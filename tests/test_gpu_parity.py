@@ -649,3 +649,17 @@ def test_forward_with_values_that_are_not_finite(D, w2):
         assert float((o.float() - want.float())[fin].abs().max()) <= 3e-2, (name, value)      # two bf16-rounded results
         if value == -math.inf:
             assert bool(fin.all()) and float((lse - want_lse).abs().max()) <= 2e-2
+
+
+@pytest.mark.parametrize("N,H,Hkv,D,w1,w2", [(1100, 8, 8, 64, 64, 4), (1100, 8, 8, 64, 64, 16), (1000, 8, 8, 128, 40, 100), (1300, 16, 4, 128, 20, 100),
+                                             (1300, 12, 12, 64, 30, 32)])
+def test_row_kernel_beside_or_after_the_column_kernel(N, H, Hkv, D, w1, w2):
+    """Where the row kernel runs (beside the column kernel, on the multiprocessors that leaves, or after it) does not touch the
+    results: a call for all gradients equals two calls for those of either kernel, bit for bit."""
+    ts = so.make_inputs(1, N, H, Hkv, D, seed=61, seed_do=62)
+    cfg = dict(w1=w1, w2=w2, scale=1.0 / math.sqrt(D), k2_bias=0.0, v2_bias=0.0)
+    ins = dict(zip(("q", "k1", "k2", "v1", "v2", "do"), ts))
+    whole = _run(ins, cfg, "tcgen05")[2]
+    col, row = _run(ins, cfg, "tcgen05", need=(False, True, False, True, False))[2], _run(ins, cfg, "tcgen05", need=(True, False, True, False, True))[2]
+    for i, other in ((0, row), (1, col), (2, row), (3, col), (4, row)):
+        assert bool(torch.isfinite(whole[i]).all()) and torch.equal(whole[i], other[i]), i
