@@ -563,7 +563,11 @@ int sa_forward_status(const sa_params* p, const void* q, const void* k1, const v
         if (p->algo == SA_ALGO_TCGEN05) return SA_ERR_BAD_STRIDE;
         algo = SA_ALGO_GENERAL;
     }
-    if (algo == SA_ALGO_TCGEN05) return launch_fwd_tc(p, k, q, k1, k2, v1, v2, o, lse, workspace, status, st);
+    if (algo == SA_ALGO_TCGEN05) {
+        // (BAD_STRIDE: a tensor map cannot hold a stride, for instance a negative one; nothing has been launched then)
+        const int rc = launch_fwd_tc(p, k, q, k1, k2, v1, v2, o, lse, workspace, status, st);
+        if (rc != SA_ERR_BAD_STRIDE || p->algo == SA_ALGO_TCGEN05) return rc;
+    }
     const cudaError_t e = sa::general::launch_fwd(p->dtype, k, q, k1, k2, v1, v2, o, lse, device_info().sm_count, st);
     g_launches += 1;
     return e == cudaSuccess ? SA_OK : SA_ERR_LAUNCH;

@@ -663,3 +663,39 @@ def test_row_kernel_beside_or_after_the_column_kernel(N, H, Hkv, D, w1, w2):
     col, row = _run(ins, cfg, "tcgen05", need=(False, True, False, True, False))[2], _run(ins, cfg, "tcgen05", need=(True, False, True, False, True))[2]
     for i, other in ((0, row), (1, col), (2, row), (3, col), (4, row)):
         assert bool(torch.isfinite(whole[i]).all()) and torch.equal(whole[i], other[i]), i
+
+
+@pytest.mark.parametrize("name", ["q", "k1", "k2", "v1", "v2", "do"])
+@pytest.mark.parametrize("dim", [0, 1, 2])
+def test_expanded_inputs(name, dim):
+    """An input that is expanded (stride 0) over the batch, the rows or the heads gives what its copy gives."""
+    B, N, H, D, w1, w2 = 2, 150, 2, 64, 50, 24
+    ts = {nm: t.to(DEV).to(torch.bfloat16) for nm, t in zip(("q", "k1", "k2", "v1", "v2", "do"), so.make_inputs(B, N, H, H, D, seed=71, seed_do=72))}
+    ts[name] = ts[name].narrow(dim, 0, 1).expand_as(ts[name])
+
+    def both(t):
+        o, lse = sab.two_simplicial_attn_fwd_kernel(*(t[nm] for nm in ("q", "k1", "k2", "v1", "v2")), w1, w2, 0.125, algo="tcgen05")
+        return (o, lse) + sab.two_simplicial_attn_bwd(*(t[nm] for nm in ("q", "k1", "k2", "v1", "v2")), o, lse, t["do"], w1, w2, 0.125)
+
+    for a, b in zip(both(ts), both(dict(ts, **{name: ts[name].contiguous()}))):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["q", "k2", "v2", "k1"])
+def test_forward_with_rows_in_reverse_order(name):
+    """A negative row stride, which a tensor map does not hold, takes the general kernels."""
+    B, N, H, D, w1, w2 = 1, 150, 2, 64, 50, 24
+    names = ("q", "k1", "k2", "v1", "v2")
+    ts = {nm: t.to(DEV).to(torch.bfloat16) for nm, t in zip(names, so.make_inputs(B, N, H, H, D, seed=73, seed_do=74))}
+    want, want_lse = sab.two_simplicial_attn_fwd_kernel(*(ts[nm] for nm in names), w1, w2, 0.125)
+    back = ts[name].flip(1).contiguous()
+    o, lse = torch.empty_like(want), torch.empty_like(want_lse)
+    p = host._make_params(*(ts[nm] for nm in names), o, w1, w2, 0.125, 0.0, 0.0, 0, 0, "auto")
+    setattr(p, name, _abi.Strides(back.stride(0), -back.stride(1), back.stride(2)))
+    ptr = {nm: t.data_ptr() for nm, t in ts.items()}
+    ptr[name] = back[:, N - 1:].data_ptr()
+    ws = torch.zeros(256, dtype=torch.uint8, device=DEV)
+    rc = _abi.load().sa_forward(ctypes.byref(p), *(ctypes.c_void_p(ptr[nm]) for nm in names), host._ptr(o), host._ptr(lse), host._ptr(ws), ws.numel(),
+                                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == _abi.SA_OK
+    assert float((o.float() - want.float()).abs().max()) <= 3e-2 and float((lse - want_lse).abs().max()) <= 1e-2      # (two bf16-rounded results)
