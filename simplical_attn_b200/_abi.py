@@ -1,7 +1,7 @@
 """ctypes binding of libsimplicial_attn_b200.so (declarations: include/simplicial_attn_b200.h).
 
-This is the only place the Python layer touches native code.  There is no fallback: if the
-library has not been built, importing this module raises.
+This is the only place the Python layer touches native code.  There is no fallback for the library: where it has not been
+built and cannot be, `load()` raises.
 """
 from __future__ import annotations
 

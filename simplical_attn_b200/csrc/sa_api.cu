@@ -238,7 +238,6 @@ void launch_add_rows(void* dst, const sa_strides& sd, const void* tmp, int B, in
 struct DeviceInfo {
     int sm_count = 0;
     int cc_major = 0;
-    bool attrs_set = false;
 };
 
 DeviceInfo& device_info() {
@@ -321,7 +320,7 @@ int launch_fwd_tc_t(const KParams& k, const void* q, const void* k1, const void*
     P.wait_limit_ns = g_wait_limit_ns.load();
     const bool has_bias = k.k2_bias != 0.f || k.v2_bias != 0.f;
     auto go = [&](auto fn) { return fn(P, dev.sm_count, q, k1, k2, v1, v2, o, lse, st); };
-    if (k.D > 64) return has_bias ? go(launch_fwd_tc_k<128, true, F16>) : go(launch_fwd_tc_k<128, false, F16>);
+    if (k.D == 128) return has_bias ? go(launch_fwd_tc_k<128, true, F16>) : go(launch_fwd_tc_k<128, false, F16>);
     return has_bias ? go(launch_fwd_tc_k<64, true, F16>) : go(launch_fwd_tc_k<64, false, F16>);
 }
 
@@ -423,7 +422,7 @@ int resolve(const sa_params* p, bool backward) {
 
 extern "C" {
 
-int sa_version(void) { return 200; }
+int sa_version(void) { return 300; }
 
 uint64_t sa_kernel_launches(void) { return g_launches.load(); }
 

@@ -220,10 +220,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
-// Arrives without waiting: the barrier completes once `nthreads` threads have arrived or synchronised on it.
-__device__ __forceinline__ void named_barrier_arrive(int id, int nthreads) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 
 // ----------------------------------------------------------------------------------------------
 // TMA (tiled, 4-d, global -> shared, completion on an mbarrier)
@@ -361,31 +357,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]
         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-
-// N columns of the thread's own lane (N = 16 or 32), N packed words (8 or 16).
-template <int N>
-__device__ __forceinline__ void tmem_ld_n(uint32_t addr, uint32_t (&v)[N]) {
-    static_assert(N == 16 || N == 32, "widths the softmax uses");
-    if constexpr (N == 16) tmem_ld16(addr, v);
-    else tmem_ld32(addr, v);
-}
-template <int N>
-__device__ __forceinline__ void tmem_st_n(uint32_t addr, const uint32_t (&v)[N]) {
-    static_assert(N == 8 || N == 16, "widths the softmax uses");
-    if constexpr (N == 8) tmem_st8(addr, v);
-    else tmem_st16(addr, v);
-}
-
 // ----------------------------------------------------------------------------------------------
 // tcgen05.mma descriptors (bf16 operands, fp32 accumulate, 128-byte swizzled shared-memory tiles)
 //
@@ -458,8 +429,7 @@ __device__ __forceinline__ void mma_ts(uint32_t leader, uint32_t d_tmem, uint32_
         : "memory");
 }
 
-// The same with the low words of the descriptors plus a constant: the high words are constants (kDescHiK for K-major,
-// kDescHiMn), so an issuer loop holds one 32-bit register per operand instead of a 64-bit one per operand and step.
+// The same with the low words of the descriptors plus a constant: the high words are a constant (kDescHi), so an issuer loop holds one 32-bit register per operand instead of a 64-bit one per operand and step.
 constexpr uint32_t kDescHi = (uint32_t)((((uint64_t)(1024u >> 4)) << 32 | kDescVersion | kDescSwizzle128) >> 32);
 template <int OFFA, int OFFB>
 __device__ __forceinline__ void mma_ss_lo(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate) {
@@ -499,11 +469,6 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_byt
     return ((smem_addr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16);
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
 // max of three values in one instruction
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
@@ -515,12 +480,6 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-
-
-// bf16 pair held in a 32-bit word -> floats, by bit operations only (a register array reinterpreted
-// through a pointer cast tends to be demoted to local memory).
-__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // The 16-bit element type of the tensor-core kernels: bf16 (F16 = false) or IEEE half (F16 = true).  The
 // kernels move elements as raw 16-bit patterns (pointers are typed __nv_bfloat16 for their size only);
@@ -595,13 +554,8 @@ __device__ __forceinline__ uint4 mul_chunk(const uint4& xa, const uint4& ya, flo
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// With bias == 0 the product of two bf16 values rounded to bf16 is exactly what the packed bf16
-// multiply returns (the product of two 8-bit significands is exact in fp32, one rounding follows).
-__device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
+// With bias == 0 the product of two 16-bit values rounded to 16 bits is exactly what the packed multiply returns (the
+// product of two significands is exact in fp32, one rounding follows).
 template <bool F16 = false>
 __device__ __forceinline__ uint4 mul_chunk_nobias(const uint4& xa, const uint4& ya) {
     using E = El<F16>;
@@ -804,10 +758,6 @@ __device__ __forceinline__ float half_warp_transpose_reduce16(float (&v)[16], in
     return half_warp_transpose_reduce<16>(v, lane);
 }
 
-// Byte offset of element (row, col) inside a 128-byte-swizzled [rows x 64] bf16 slab.
-__device__ __forceinline__ uint32_t swz128_offset(int row, int col) {
-    return (uint32_t)row * 128u + ((((uint32_t)col >> 3) ^ ((uint32_t)row & 7u)) << 4) + (((uint32_t)col & 7u) << 1);
-}
 
 }  // namespace ptx
 }  // namespace sa

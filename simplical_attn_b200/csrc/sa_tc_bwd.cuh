@@ -270,10 +270,10 @@ struct ColSmem {
 // under dV1(t) and S(t+1), so neither side waits for a whole chain of the other.
 // Bound by the softmax groups (exponentials: 1024 cycles per tile at 16 per clock, measured 2000 with their loads,
 // stores and hand-overs, plus 880 for dS) and the issue of the SS MMAs (100 cycles each while the producers store the
-// next tiles, 64 without), 3700 cycles per tile where the whole chain per tile took 4300.  Measured, us, before ->
-// after: B1 N16384 H32/2 D128 w 512/32 11706 -> 9690; B1 N8192 H16 D128 w 1024/64 10558 -> 9010; B4 N2048 H16 D64
-// w 64/64 1449 -> 1217; B2 N512 H4 D64 w 32/32 89 -> 78; at short windows with 16 deltas, where every tile is half masked
-// and the producers set the pace, it costs: B4 N8192 H16 D128 w 128/16 2555 -> 2843 (3067 with 96 registers for them).
+// next tiles, 64 without), 3700 cycles per tile; 4300 where the whole chain is walked per tile.  dK1 and dV1 alone, us,
+// by a chain per tile and so: B1 N2048 H8/1 D64 w 512/64 4757 and 4123, w 64/32 808 and 689, w 64/16 449 and 379;
+// B1 N8192 H16 D128 w 1024/64 10558 and 9150; where the producers set the pace it costs: w2 = 8 (operand rows formed one by
+// one) 1340 and 1471, B4 N8192 H16 D128 w 128/16 (every tile half masked) 2555 and 2850.
 // Registers per thread of the column kernel's softmax groups, producers and remaining warps (multiples of 8).
 #ifndef SA_COL_SM
 #define SA_COL_SM 112

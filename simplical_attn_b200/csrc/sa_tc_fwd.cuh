@@ -25,7 +25,8 @@
 // The row tiles work in opposite phase: while one is in its softmax the tensor cores work for the other.  Column tiles
 // are 128 wide because an MMA of 128 x 64 x 16 with A in shared memory takes 48 cycles, one of 128 x 128 x 16 takes 64:
 // per row tile and 128 columns 1024 cycles of MMA instead of 1280.  The exponentials take another 1024 (16 per clock
-// for the multiprocessor), so both units are at best half idle only while waiting for each other's hand-overs.
+// for the multiprocessor).  A pair of row tiles takes about 5600 cycles per 128 columns, so neither unit is the limit but
+// the chain S -> softmax -> P -> P.V of each row tile with its hand-overs.
 // Tensor memory: S0 | S1 (128 columns each, P overwrites S in place as packed 16-bit values) | T0 | T1 (D columns).
 #pragma once
 
@@ -65,7 +66,7 @@ struct FwdTcParams {
     uint64_t wait_limit_ns;   // bound of every device-side wait
 };
 
-// Shared memory: fixed part, A tiles, K1 ring, V1 ring, raw K2 / V2 window rows and Q rows of a unit.
+// Shared memory: fixed part, A tiles, ring of K1 and V1 buffers, raw K2 / V2 window rows and Q rows of a unit.
 template <int HD>
 struct FwdSmem {
     static constexpr int kSlabs = HD / 64;                       // 64-element slabs per tile
@@ -161,8 +162,7 @@ struct RingPos {
 };
 
 // BIAS = false: both biases are zero, every bias add folds away.  F16: the tensors are IEEE half instead of bf16
-// (same kernels; only the element encoding and the MMA's operand format differ).  The head dim may be smaller than
-// HD (a multiple of 8): TMA fills the missing columns with zeros and they are not written out.
+// (same kernels; only the element encoding and the MMA's operand format differ).
 template <int HD, bool BIAS, bool F16 = false>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUtensorMap map_k1,
@@ -530,7 +530,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                     halve(4, std::integral_constant<int, 2>{});
                     if (CLS == 2 && P.dw_log2 >= 6)
                         asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(part + (wq * HD + 64 * ch + 2 * lane) * 4), "f"(acc[0]), "f"(acc[1]) : "memory");
-                    else if (i < p.N && 64 * ch + 2 * lane < p.D)
+                    else if (i < p.N)
                         *(uint32_t*)(orow + 2 * lane) = E::pack(acc[0], acc[1]);
                 } else {
                     // four rows to a query: lanes t/4 = 0..3 and 4..7 hold different ones
@@ -538,8 +538,8 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                     halve(4, std::integral_constant<int, 4>{});
                     const int col = 16 * ((lane >> 2) & 3) + 2 * (lane & 3);
                     if (i < p.N) {
-                        if (64 * ch + col < p.D) *(uint32_t*)(orow + col) = E::pack(acc[0], acc[1]);
-                        if (64 * ch + col + 8 < p.D) *(uint32_t*)(orow + col + 8) = E::pack(acc[2], acc[3]);
+                        *(uint32_t*)(orow + col) = E::pack(acc[0], acc[1]);
+                        *(uint32_t*)(orow + col + 8) = E::pack(acc[2], acc[3]);
                     }
                 }
 #pragma unroll
@@ -589,7 +589,7 @@ fwd_tc_kernel(const __grid_constant__ FwdTcParams P, const __grid_constant__ CUt
                     const int q2 = idx / HD, col = idx % HD, i = i0 + q2;
                     float sum = 0.f;
                     for (int w = 0; w < wpq; ++w) sum += lds_f32(part + ((q2 * wpq + w) * HD + col) * 4);
-                    if (i < p.N && col < p.D) E::st(obase + (long)i * p.o.n + col, sum);
+                    if (i < p.N) E::st(obase + (long)i * p.o.n + col, sum);
                 }
                 named_barrier_sync(1 + r, 128);
             }
