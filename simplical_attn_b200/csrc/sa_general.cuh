@@ -632,22 +632,24 @@ inline int col_cluster(const KParams& p, int sm_count) {
     return nrank;
 }
 
-// Tiles or a warp per output row: the smaller of two estimates, in us, with constants measured on a B200 over 437 problems
-// (head dims 32, 64, 128, 256, windows 1 ... 1024 / 1 ... 160, sequences of 1 ... 4096 rows): the faster of the two kernels within
-// 5 % in 95 % of them, at worst 0.53 of its speed (a few short launches).
-//   rows:  0.14 R + (pairs + outer o) max(0.32, pair R), with R output rows (warps) per multiprocessor, a row's (j, k) pairs
-//          and outer steps (K2 rows, or for dK1/dV1 queries);
-//   tiles: max(1.75, blocks per multiprocessor) x (passes x (tile + group x 16-column groups)), for dK1/dV1
-//          (tile + group x tiles).
+// Tiles or a warp per output row: the smaller of two estimates, in us, with constants measured on a B200 over 637 problems
+// (head dims 8 ... 256, windows 1 ... 1024 / 1 ... 160, sequences of 1 ... 4096 rows, among them 200 of the usual sizes): the
+// faster of the two kernels within 5 % in 95 % of them, at worst 0.59 of its speed (short launches).
+//   rows:  0.14 R + max(wait (pairs + o outer) of the longest row, pair R (pairs + o outer) of the mean row), with R output
+//          rows (warps) per multiprocessor, a row's (j, k) pairs and outer steps (K2 rows, or for dK1/dV1 queries);
+//   tiles: max(first, blocks per multiprocessor) x (passes x (tile + group x 16-column groups)), for dK1/dV1
+//          (tile + group x tiles), where `first` is what a launch of few blocks takes.
+// Long windows always go by tiles: no warp per row was measured to be the faster one there, and the estimate does not
+// hold for them (their rows no longer stay in the caches).
 enum Kernel { kFwd = 0, kDq = 1, kKv1 = 2, kKv2 = 3 };
 struct Cost {
-    double pair[4], o, tile[4], group[4];      // by padded head dim 32, 64, 128, 256
+    double pair[4], o, wait, tile[4], group[4];      // [4]: by padded head dim 32, 64, 128, 256
 };
 constexpr Cost kCost[4] = {
-    {{.013, .013, .019, .028}, .5, {3.8, 5.4, 18, 25}, {.97, 1.4, 2.6, 6.8}},
-    {{.013, .013, .017, .031}, .68, {3.5, 6.6, 20, 34}, {1.3, 1.8, 3.5, 9.2}},
-    {{.013, .014, .021, .086}, 1.2, {2.5, 2.5, 0, 0}, {4.8, 8.1, 21, 45}},
-    {{.013, .015, .020, .039}, 1.5, {3.6, 11, 21, 37}, {1.5, 2.7, 4.6, 12}},
+    {{.013, .013, .019, .030}, .48, .28, {4.3, 6.1, 19, 27}, {.72, 1.1, 2.0, 5.4}},
+    {{.013, .014, .018, .032}, .71, .27, {4.1, 7.5, 21, 38}, {.93, 1.4, 2.8, 7.5}},
+    {{.013, .015, .022, .079}, 1.7, .24, {3.0, 3.3, 10, 12}, {4.6, 7.8, 20, 44}},
+    {{.013, .016, .021, .051}, 1.7, .25, {4.5, 13, 23, 44}, {1.3, 2.2, 4.1, 10}},
 };
 
 // K1 (K2) rows that a query sees, averaged over the queries: windows are cut at the first row that exists.
@@ -661,9 +663,11 @@ inline bool by_rows(Kernel kernel, const KParams& p, int sm_count) {
     const int d = p.D <= 32 ? 0 : p.D <= 64 ? 1 : p.D <= 128 ? 2 : 3;
     const int n_out = kernel == kKv1 ? p.n1 : kernel == kKv2 ? p.n2 : p.N;
     const double heads = kernel < kKv1 ? p.H : p.Hkv, group = kernel < kKv1 ? 1 : p.G;
+    if ((double)p.w1 * p.w2 > 3300 || (kernel == kKv1 && p.w1 > 24)) return false;
     const double m1 = mean_window(p, p.w1, p.halo1), m2 = mean_window(p, p.w2, p.halo2), per = group * p.N / n_out;
     const double warps = p.B * heads * n_out / sm_count;
-    const double rows = .14 * warps + per * (m1 * m2 + c.o * (kernel == kKv1 ? m1 : m2)) * fmax(.32, c.pair[d] * warps);
+    const double longest = c.wait * group * ((double)p.w1 * p.w2 + c.o * (kernel == kKv1 ? p.w1 : p.w2));
+    const double rows = .14 * warps + fmax(longest, c.pair[d] * warps * per * (m1 * m2 + c.o * (kernel == kKv1 ? m1 : m2)));
     double blocks, tiles;
     if (kernel == kKv1) {
         const int nrank = col_cluster(p, sm_count);
@@ -675,7 +679,7 @@ inline bool by_rows(Kernel kernel, const KParams& p, int sm_count) {
         blocks = p.B * heads * ((n_out + owners - 1) / owners);
         tiles = group * ((p.w2 + kRows - 1) / kRows) * (c.tile[d] + c.group[d] * (((span < p.n1 ? span : p.n1) + 15) / 16));
     }
-    return rows <= fmax(1.75, blocks / sm_count) * tiles;
+    return rows <= fmax(d < 2 ? 1.75 : 1, blocks / sm_count) * tiles;
 }
 
 template <typename T, int DP>

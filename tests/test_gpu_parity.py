@@ -510,6 +510,8 @@ GENERAL_CASES = [
     (1, 130, 2, 2, 8, 100, 5, 0.0, 0.0, 3, 2),
     (2, 70, 2, 1, 100, 6, 5, 0.0, 0.1, 0, 0),
     (4, 40, 2, 2, 64, 3, 3, 0.1, 0.0, 2, 2),
+    (2, 60, 1, 1, 200, 10, 3, 0.0, 0.0, 0, 0),
+    (2, 50, 2, 2, 20, 3, 2, 0.0, 0.0, 0, 0),
 ]
 
 
