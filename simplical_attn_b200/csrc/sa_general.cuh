@@ -124,14 +124,15 @@ __device__ __forceinline__ void row_stats(float* delta, float* L, const int* ri,
 
 // s[a][c] = X[4 ty + a] . Y[tx + 16 c], summed in blocks of 16 products: a single chain over the head dim made the error of
 // dQ and dK2 against 64 bits larger than the row kernels' (fp32 D128 w 100/40: 6.6e-7 and 6.9e-7 against 5.6e-7 and 6.1e-7).
-template <int DP, int NC>
+// UNROLL blocks are unrolled: more than one spills where NC is 4.
+template <int DP, int NC, int UNROLL = 1>
 __device__ __forceinline__ void product(const float* X, const float* Y, int ty, int tx, float (&s)[4][NC]) {
     constexpr int P = Shape<DP>::kPitch;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int c = 0; c < NC; ++c) s[a][c] = 0.f;
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int d0 = 0; d0 < DP; d0 += 16) {
         float t[4][NC];
 #pragma unroll
@@ -542,8 +543,8 @@ bwd_col_kernel(KParams p, const T* __restrict__ q, const T* __restrict__ k1, con
         });
         const bool check = __syncthreads_or(bad);
         float s[4][NC], dp[4][NC];
-        product<DP, NC>(As, Ks, ty, tx, s);
-        product<DP, NC>(Cs, Vs, ty, tx, dp);
+        product<DP, NC, 4>(As, Ks, ty, tx, s);
+        product<DP, NC, 4>(Cs, Vs, ty, tx, dp);
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             int lo, hi;
